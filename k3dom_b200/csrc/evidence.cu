@@ -18,8 +18,9 @@
 // within a tile immaterial); DS keeps a tile's rays in input order (a stable sort by tile), as
 // its first-100 rule needs. One CTA takes one (tile, chunk of rays) work item
 // from a device work counter and stages the chunk's rays in shared memory; its warps pull the
-// tile's 4x4x2-cell sub-blocks from a block-local counter, cull 32 rays at a time with one
-// ballot, and every lane evaluates the surviving rays for its own cell.
+// tile's 4x4x2-cell sub-blocks from a block-local counter and cull 32 rays at a time with one
+// ballot. K3DOM collects the surviving rays into batches of 32, resolves them in FP64 and evaluates
+// two rays at a time for four cells per lane; DS evaluates each ray for every lane's own cell.
 //
 // K3DOM evidence is summed in fixed point: each kernel value is rounded once to an integer
 // number of units of 2^-k sigma (the table carries the scale), summed exactly in 64-bit
@@ -46,9 +47,9 @@ constexpr int kKernelTabEntries = kKernelTab + 1;  // + a zero entry at u = 1
 static_assert(kKernelTabEntries == kKernelTableSize, "kernel table size");
 constexpr int kEvThreads = 256;
 constexpr int kEvWarps = kEvThreads / 32;
-constexpr int kSmallChunk = 256;  // items up to this many rays run in CTAs of kSmallWarps warps
-constexpr int kSmallWarps = 4;
+constexpr int kEvCtas = 4;  // K3DOM evidence CTAs per SM: 64 registers a thread
 constexpr int kDsMaxNeighbors = 100;  // measurement_grid.cu:87
+constexpr int kFxShift = 40;  // fixed-point units of the K3DOM and calibration sums: 2^-40 of the scaled kernel
 
 // ================================================================ binning
 struct BinGeom {
@@ -509,12 +510,13 @@ void fill_scene_evidence(SceneDev& sd, bool ds, float4* ktab) {
         rls = sqrtf(p.window_radius * p.window_radius + slack) + 1e-3f * p.res;
     }
     sd.cull_ls2 = rls * rls;
-    // fixed point: one kernel value is at most sigma -> at most 2^40 units, leaving 2^23 terms
-    // of headroom in a signed 64-bit sum
+    // fixed point: the table is scaled by a power of two so that a kernel value is at most 1, and
+    // one unit is 2^-40 of that: at most 2^40 units a value, leaving 2^23 terms of headroom in a
+    // signed 64-bit sum
     const double sig = std::max((double)p.sigma, 1e-30);
-    const int sh = 40 - (int)std::ceil(std::log2(sig));
+    const int sh = kFxShift - (int)std::ceil(std::log2(sig));
     sd.fx_inv = std::ldexp(1.0, -sh);
-    if (ktab) build_kernel_table(p.sigma, std::ldexp(1.0, sh), ktab);
+    if (ktab) build_kernel_table(p.sigma, std::ldexp(1.0, sh - kFxShift), ktab);
 }
 
 // Worst case of tiles one ray can reach: for each slab of tiles along the ray's dominant axis A,
@@ -613,6 +615,16 @@ __device__ __forceinline__ void centre_xyz(int ix, int iy, int iz, const DevPara
     *z = __fsub_rn(__fmul_rn(__fsub_rn(__fadd_rn((float)iz, 0.5f), hz), p.res), sz);
 }
 
+// First cell (of the lowest indices) of sub-block sb in tile t.
+struct SbCell {
+    int x, y, z;
+};
+__device__ __forceinline__ SbCell sb_cell(const TileShape& ts, int t, int sb) {
+    const int tx = t % ts.ntx, ty = (t / ts.ntx) % ts.nty, tz = t / (ts.ntx * ts.nty);
+    const int sbx = sb % ts.nsbx, sby = (sb / ts.nsbx) % ts.nsby, sbz = sb / (ts.nsbx * ts.nsby);
+    return SbCell{tx * ts.tx + sbx * 4, ty * ts.ty + sby * 4, tz * ts.tz + sbz * 2};
+}
+
 __device__ __forceinline__ CellLoc locate(const DevParams& p, const TileShape& ts, int t, int sb, int lane,
                                           float sx, float sy, float sz) {
     const int tx = t % ts.ntx, ty = (t / ts.ntx) % ts.nty, tz = t / (ts.ntx * ts.nty);
@@ -646,10 +658,9 @@ __device__ __forceinline__ void sb_order_keys(SbOrder& o, const DevParams& p, co
                                               float sx, float sy, float sz) {
     const int i = threadIdx.x;
     if (nsb > kMaxOrderedSb || i >= nsb) return;
-    const int tx = t % ts.ntx, ty = (t / ts.ntx) % ts.nty, tz = t / (ts.ntx * ts.nty);
-    const int sbx = i % ts.nsbx, sby = (i / ts.nsbx) % ts.nsby, sbz = i / (ts.nsbx * ts.nsby);
+    const SbCell b = sb_cell(ts, t, i);
     float x, y, z;
-    centre_xyz(tx * ts.tx + sbx * 4 + 2, ty * ts.ty + sby * 4 + 2, tz * ts.tz + sbz * 2 + 1, p, sx, sy, sz, &x, &y, &z);
+    centre_xyz(b.x + 2, b.y + 2, b.z + 1, p, sx, sy, sz, &x, &y, &z);
     o.key[i] = x * x + y * y + z * z;
 }
 
@@ -749,24 +760,6 @@ struct TabPos {
     int i;
     float f;
 };
-__device__ __forceinline__ TabPos tab_pos(float t) {
-    const float tr = __fadd_rd(t, 8388608.0f);
-    TabPos q;
-    q.i = __float_as_int(tr) - 0x4B000000;
-    q.f = t - (tr - 8388608.0f);
-    return q;
-}
-__device__ __forceinline__ float tab_eval(const float4* __restrict__ tab, TabPos q) {
-    const float4 c = tab[q.i];
-    return fmaf(q.f, fmaf(q.f, fmaf(q.f, c.w, c.z), c.y), c.x);
-}
-__device__ __forceinline__ float tab_eval_tex(cudaTextureObject_t tab, int base, TabPos q) {
-    const float4 c = tex1Dfetch<float4>(tab, base + q.i);
-    return fmaf(q.f, fmaf(q.f, fmaf(q.f, c.w, c.z), c.y), c.x);
-}
-__device__ __forceinline__ float kernel_tab(const float4* __restrict__ tab, float t) {
-    return tab_eval(tab, tab_pos(t));
-}
 
 // mass_update.cu:12-14, 1 - 2 / (1 + exp(2 mass / mass_scale)), with k2 = 2 / mass_scale
 __device__ __forceinline__ double calc_credit(double mass, double k2) {
@@ -881,16 +874,15 @@ __device__ __forceinline__ void k3dom_cell_update(const DevParams& p, double g, 
     k3dom_cell_update_in(p, g, c, del_occ, del_free, load_cell_in(cs, cw, c, first_frame), cs, cw, first_frame);
 }
 
-// Shared memory of k_bgki: one chunk of rays and a per-warp staging area for the FP64
-// (sub-block, ray) constants of the rays that pass the cull. (The kernel table is read through
-// the texture path: its lanes' scattered 16-byte reads ran 10 % slower from shared memory,
-// where they conflicted on banks and queued behind the staging loads.)
-// (dynamic, sized by the work item's ray count so that smaller chunks leave room for more CTAs)
+// Shared memory of the evidence kernels: one chunk of rays (the cull's constants; the FP64 ones are
+// read from global memory for the candidates only), the per-warp candidate rings and pair records.
+// Dynamic, sized by the largest work item's ray count.
 struct BgkiSmem {
-    float* stage;                 // [warps][kStageWarpFloats] pair records of the passing rays
-    float4* a;                    // [chunk] m.x, m.y, m.z, d_m
-    double4* c;                   // [chunk] d_m, margin, 1/d_m
-    uint16_t* reg;                // [kRegions][chunk] rays per region of a 16x16 tile (region builds)
+    float* stage;    // [warps][kStageWarpFloats] pair records of the candidate rays
+    uint16_t* ring;  // [warps][2][kRing] candidate rays waiting for a full batch: interior, general
+    float4* u;       // [chunk] m / d_m, d_m
+    uint32_t* rid;   // [chunk] point slot
+    uint16_t* reg;   // [kRegions][chunk] rays per region of a 16x16 tile
 };
 
 // A 16x16-cell tile splits into kRegions columns of 8x8 cells (full tile height); a ray's region
@@ -901,30 +893,30 @@ constexpr int kRegions = 4;
 
 // A pair record holds the staged constants of two rays a, b interleaved per component, so that one
 // 8-byte register pair feeds a packed instruction:
-//   float4 0: (perp0.x, perp0.y) of a, b     1: (perp0.z, par0)
-//   float4 2: (u.x, u.y)                     3: (u.z, par0 - margin)
-//   float4 4: (occ0.x, occ0.y)               5: (occ0.z, par0 - d_m)
-// each float4 as (a, b, a, b); a seventh float4 pads the record so that the 32 lanes' scalar
-// stores spread over the banks.
-constexpr int kStagePairFloats = 28;
-constexpr int kStageWarpFloats = 16 * kStagePairFloats;
+//   float4 0: (perp0.x, perp0.y) of a, b     1: (perp0.z, u.x)     2: (u.y, u.z)
+// and, in the records of near and edge rays,
+//   float4 3: (par0, par0 - margin)          4: (occ0.x, occ0.y)   5: (occ0.z, par0 - d_m)
+// each float4 as (a, b, a, b); the larger records are padded by a seventh float4 so that the four
+// records a step reads lie in different banks (12 floats do without).
+constexpr int kRecInterior = 12, kRecGeneral = 28;
+constexpr int kStageWarpFloats = 16 * kRecGeneral;
+constexpr int kRing = 64;  // candidates kept per warp and class: up to 31 waiting and 32 new ones
 
-__host__ __device__ constexpr size_t bgki_fixed_bytes(int warps) {
-    return (sizeof(float) * (size_t)warps * kStageWarpFloats + 31) & ~(size_t)31;
+constexpr size_t kBgkiFixedBytes = (size_t)kEvWarps * (sizeof(float) * kStageWarpFloats + 2 * sizeof(uint16_t) * kRing);
+static_assert(kBgkiFixedBytes % 32 == 0, "alignment of what follows");
+
+inline size_t bgki_smem_bytes(int chunk) {
+    return kBgkiFixedBytes +
+           (size_t)chunk * (sizeof(float4) + sizeof(uint32_t) + kRegions * sizeof(uint16_t));
 }
 
-inline size_t bgki_smem_bytes(int chunk, int warps = kEvWarps, bool regions = false) {
-    return bgki_fixed_bytes(warps) + (size_t)chunk * (sizeof(float4) + sizeof(double4)) +
-           (regions ? (size_t)kRegions * chunk * sizeof(uint16_t) : 0);
-}
-
-__device__ __forceinline__ BgkiSmem bgki_smem(unsigned char* base, int chunk, int warps) {
+__device__ __forceinline__ BgkiSmem bgki_smem(unsigned char* base, int chunk) {
     BgkiSmem S;
     S.stage = reinterpret_cast<float*>(base);
-    const size_t off = bgki_fixed_bytes(warps);
-    S.c = reinterpret_cast<double4*>(base + off);  // 32-byte aligned
-    S.a = reinterpret_cast<float4*>(base + off + sizeof(double4) * (size_t)chunk);
-    S.reg = reinterpret_cast<uint16_t*>(base + off + (sizeof(double4) + sizeof(float4)) * (size_t)chunk);
+    S.ring = reinterpret_cast<uint16_t*>(base + sizeof(float) * (size_t)kEvWarps * kStageWarpFloats);
+    S.u = reinterpret_cast<float4*>(base + kBgkiFixedBytes);
+    S.rid = reinterpret_cast<uint32_t*>(S.u + chunk);
+    S.reg = reinterpret_cast<uint16_t*>(S.rid + chunk);
     return S;
 }
 
@@ -965,35 +957,99 @@ __device__ __forceinline__ unsigned region_mask(float ax, float ay, float az, fl
     return q;
 }
 
-// Stages the item's rays (m, d_m) and FP64 constants in shared memory and, for a 16x16 tile,
-// appends each ray to the lists of the regions it reaches (rcnt zeroed before the call; list
-// order is arbitrary, the sums are exact). Every thread of the block calls it.
-template <int THREADS>
-__device__ __forceinline__ void stage_item_rays(const EvArgs& A, const Item& it, const SceneDev& sd,
-                                                const FrameParams& fp, bool regions, float4* sa, double4* sc,
-                                                uint16_t* reg, int* rcnt) {
-    const DevParams& p = sd.p;
-    const TileShape& ts = sd.ts;
+// What the warps of a CTA need of the work item they hold, in shared memory: kept in registers it
+// would crowd out the evaluation loops' own values at 64 registers a thread.
+struct ItemConst {
+    int live;  // 0: no item left
+    int t, lt, nr, nsb, regions, coff, tbase;
+    uint32_t e0, n_items;
+    TileShape ts;
+    int sc, G, Gz;
+    float res, sx, sy, sz;
+    float bin_R, ls2, tscale, rls2, rls;
+};
+
+// Takes the next work item (the calling warp only).
+__device__ __forceinline__ void fetch_item(const EvArgs& A, uint32_t total_items, int chunk, ItemConst* I) {
+    const Batch& bt = A.bt;
+    const int lane = threadIdx.x & 31;
+    uint32_t item = 0;
+    if (lane == 0) item = atomicAdd(&A.status->work_counter, 1u);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    if (item >= total_items) {
+        if (lane == 0) I->live = 0;
+        return;
+    }
+    // the tile: last t with item_off[t] <= item, 32 probes a step
+    int lo = 0, hi = bt.T;
+    while (hi - lo > 1) {
+        const int span = hi - lo;
+        const int pos = span <= 33 ? min(lo + 1 + lane, hi) : lo + (int)((long)(lane + 1) * span / 33);
+        const unsigned m = __ballot_sync(0xffffffffu, pos < hi && A.item_off[pos] <= item);
+        const int n = __popc(m);  // a prefix of the lanes
+        const int at = __shfl_sync(0xffffffffu, pos, n > 0 ? n - 1 : 0);
+        const int up = __shfl_sync(0xffffffffu, pos, n < 32 ? n : 31);
+        if (n > 0) lo = at;
+        if (n < 32) hi = min(hi, up);
+    }
+    if (lane != 0) return;
+    I->live = 1;
+    I->t = lo;
+    I->sc = scene_of(bt.off->tile, bt.S, lo);
+    I->lt = lo - bt.off->tile[I->sc];
+    const uint32_t first = A.item_off[lo];
+    I->n_items = A.item_off[lo + 1] - first;
+    I->e0 = A.tile_start[lo] + (item - first) * (uint32_t)chunk;
+    const uint32_t e1 = min(A.tile_start[lo + 1], I->e0 + (uint32_t)chunk);
+    I->nr = (int)(e1 > I->e0 ? e1 - I->e0 : 0);
+    const SceneDev& sd = bt.sc[I->sc];
+    const FrameParams& fp = bt.fp[I->sc];
+    const TileShape ts = sd.ts;
+    I->ts = ts;
+    I->nsb = ts.nsbx * ts.nsby * (ts.tz / 2);
+    I->regions = ts.tx == 16 && ts.ty == 16;
+    I->coff = bt.off->cell[I->sc];
+    I->tbase = I->sc * kKernelTabEntries;
+    I->G = sd.p.G;
+    I->Gz = sd.p.Gz;
+    I->res = sd.p.res;
+    I->sx = fp.sensor_x;
+    I->sy = fp.sensor_y;
+    I->sz = fp.sensor_z;
+    I->bin_R = sd.bin_R;
+    const float ls2 = sd.p.ls * sd.p.ls;
+    I->ls2 = ls2;
+    I->tscale = (1.0f / ls2) * (float)kKernelTab;  // d^2 -> table position
+    I->rls2 = sd.cull_ls2;
+    I->rls = sqrtf(sd.cull_ls2);
+}
+
+// Stages the item's rays in shared memory and, for a 16x16 tile, appends each ray to the lists of
+// the regions it reaches (rcnt zeroed before the call; list order is arbitrary, the sums are
+// exact). Every thread of the block calls it.
+__device__ __forceinline__ void stage_item_rays(const EvArgs& A, const ItemConst& I, const BgkiSmem& S, int* rcnt) {
     const int lane = threadIdx.x & 31;
     const unsigned lanes_below = (1u << lane) - 1u;
-    BinGeom g;
-    place_sensor(g, p, fp);
-    const float x0 = (float)(it.lt % ts.ntx * 16), y0 = (float)((it.lt / ts.ntx) % ts.nty * 16);
-    const float z0 = (float)(it.lt / (ts.ntx * ts.nty) * ts.tz);
-    for (int r0 = 0; r0 < it.nr; r0 += THREADS) {  // uniform trip count: the ballots below
+    const TileShape ts = I.ts;
+    const bool regions = I.regions != 0;
+    const int nr = I.nr;
+    // the sensor in cell-index space (place_sensor)
+    const float hg = (float)I.G / 2.0f, hz = (float)I.Gz / 2.0f, ir = 1.0f / I.res;
+    const float ax = I.sx / I.res + hg - 0.5f, ay = I.sy / I.res + hg - 0.5f, az = I.sz / I.res + hz - 0.5f;
+    const float x0 = (float)(I.lt % ts.ntx * 16), y0 = (float)((I.lt / ts.ntx) % ts.nty * 16);
+    const float z0 = (float)(I.lt / (ts.ntx * ts.nty) * ts.tz);
+    for (int r0 = 0; r0 < nr; r0 += kEvThreads) {  // uniform trip count: the ballots below
         const int r = r0 + (int)threadIdx.x;
         unsigned qm = 0;
-        if (r < it.nr) {
-            uint32_t rid = A.evals[it.e0 + r];
+        if (r < nr) {
+            uint32_t rid = A.evals[I.e0 + r];
             if (rid >= (uint32_t)A.bt.N) rid = 0;  // defensive: never read past the ray arrays
             const float4 a4 = A.ray_a[rid];
-            sa[r] = a4;
-            sc[r] = A.ray_c[rid];
-            if (regions) {
-                const float ir = 1.0f / p.res;  // K3DOM binning segment: sensor -> point
-                qm = region_mask(g.ax, g.ay, g.az, a4.x * ir, a4.y * ir, a4.z * ir, x0, y0, z0, ts.tz,
-                                 sd.bin_R + 0.25f);
-            }
+            const double inv = A.ray_c[rid].z;
+            S.rid[r] = rid;
+            S.u[r] = make_float4((float)(a4.x * inv), (float)(a4.y * inv), (float)(a4.z * inv), a4.w);
+            if (regions)  // K3DOM binning segment: sensor -> point
+                qm = region_mask(ax, ay, az, a4.x * ir, a4.y * ir, a4.z * ir, x0, y0, z0, ts.tz, I.bin_R + 0.25f);
         }
         if (regions) {
 #pragma unroll
@@ -1003,7 +1059,7 @@ __device__ __forceinline__ void stage_item_rays(const EvArgs& A, const Item& it,
                 int base = 0;
                 if (lane == 0) base = atomicAdd(&rcnt[q], __popc(b));
                 base = __shfl_sync(0xffffffffu, base, 0);
-                if ((qm >> q) & 1u) reg[q * A.chunk + base + __popc(b & lanes_below)] = (uint16_t)r;
+                if ((qm >> q) & 1u) S.reg[q * A.chunk + base + __popc(b & lanes_below)] = (uint16_t)r;
             }
         }
     }
@@ -1024,51 +1080,85 @@ __device__ __forceinline__ int sb_region(const TileShape& ts, int sb) {
 // Every FP32 quantity is O(ls), so the FP32 evaluation keeps ~1e-7 relative accuracy at any
 // distance from the sensor (the direct |c|^2 - d_proj^2 form of :60 loses ~1e-5 at 20 m).
 //
-// stage_pair culls the pair on the sub-block and, for a pair that passes, forms three float4:
-// st[0] = (perp0, par0), st[1] = (u, par0 - margin), st[2] = (occ0, par0 - d_m).
-//
-// The cull bounds the distance from a convex set K (the segment [0, d_m u], or the point) to the
+// The cull (cull_hits, FP32, one listed ray per lane) bounds the distance from a convex set K (the
+// segment [0, d_m u], or the point) to the
 // sub-block's cell centres x = c + h, |h_i| <= e_i, e = (1.5, 1.5, 0.5) res around the centroid c.
 // dist(K, .) is convex with gradient D / |D| at c (D = c minus the closest point of K), so
 // dist(K, x) >= |D| - (e . |D|) / |D| for every cell centre, where |D| is taken componentwise in
 // e . |D|. No cell is within rls = ls (1 + 1e-4) + 1e-3 res of K unless |D|^2 - e . |D| < rls |D|
 // (box_reaches). This is tighter than a sphere around c for the flat 4x4x2 sub-block, above all
-// for the near-horizontal rays of a LiDAR scan.
+// for the near-horizontal rays of a LiDAR scan. D is formed in FP32 from the sensor-relative
+// centroid, so rls grows by 1e-6 of the centroid's distance (about four times the rounding of the
+// products); a ray let through in excess adds nothing.
 //
-// *near: the point's sphere of radius ls can reach a cell of the sub-block. For the other rays no
-// cell of the sub-block with d_proj >= d_m is within ls of the free segment either (margin <= d_m,
-// so such a cell is at least as far from the segment's end as from the point, and the bound above
-// keeps 1e-4 ls + 1e-3 res of slack), so their free term needs no d_m test.
+// The candidates are collected over the listed rays in two warp-private rings until 32 of a class
+// are there, and only then resolved in FP64, one per lane, into pair records:
+//   interior  every cell of the sub-block projects inside [0, margin] and is farther than ls from
+//             the point: the occupied term and the along-ray term are exactly zero and are left
+//             out, as is the d_m test;
+//   general   the others: near rays (the point's sphere can reach a cell) and edge rays (a cell may
+//             project before the sensor or beyond the margin).
+// The class is decided from the cull's FP32 geometry with the same rounding slack (3 res is the most
+// a cell's own offset can add to a projection), so a ray near a limit is taken as general, which is
+// always right. Within a general batch the near rays are told apart exactly (box_reaches on the
+// point): for the others no cell with d_proj >= d_m is within ls of the free segment either (margin
+// <= d_m, so such a cell is at least as far from the segment's end as from the point, and the bound
+// above keeps 1e-4 ls + 1e-3 res of slack), so their free term needs no d_m test.
 __device__ __forceinline__ bool box_reaches(float Dx, float Dy, float Dz, float D2, float hres, float rls2) {
     const float s = fmaf(3.0f * hres, fabsf(Dx) + fabsf(Dy), hres * fabsf(Dz));
     const float t = D2 - s;
-    return t < 0.0f || t * t < rls2 * D2;
+    return t <= 0.0f || t * t < rls2 * D2;
 }
 
-__device__ __forceinline__ bool stage_pair(const float4& a, const double4& cd, double ox, double oy, double oz,
-                                           float hres, float rls2, float4 st[3], bool* near) {
+enum RayClass { kRayNone, kRayInterior, kRayGeneral };
+
+// The cull of one ray (unit direction u.xyz, length u.w) on the sub-block with centroid (cx, cy,
+// cz); rls: support radius with the rounding slack eps.
+__device__ __forceinline__ RayClass cull_ray(const float4& u, float cx, float cy, float cz, float hres, float rls,
+                                             float eps) {
+    const float proj = fmaf(cz, u.z, fmaf(cy, u.y, cx * u.x));
+    const float t = fminf(fmaxf(proj, 0.0f), u.w);
+    const float Dx = fmaf(-t, u.x, cx), Dy = fmaf(-t, u.y, cy), Dz = fmaf(-t, u.z, cz);
+    const float D2 = fmaf(Dz, Dz, fmaf(Dy, Dy, Dx * Dx));
+    if (!box_reaches(Dx, Dy, Dz, D2, hres, rls * rls)) return kRayNone;
+    // interior: proj is the centroid's projection, the anchor's lies within sqrt(3)/2 res of it, a
+    // cell's within 3 res of that
+    const float reach = 8.0f * hres + eps;
+    const float margin = fmaxf(0.9f * u.w, u.w - 4.0f * hres);
+    const float e = u.w - t, far2 = rls + 4.4f * hres;  // 4.36 hres: half diagonal of the cell centres
+    return proj > reach && margin - proj > reach && fmaf(e, e, D2) > far2 * far2 ? kRayInterior : kRayGeneral;
+}
+
+// The constants of a candidate, in the order of the pair record.
+struct RayStage {
+    float v[12];
+};
+
+__device__ __forceinline__ void stage_interior(const float4& a, double inv, const float4& u, float oxf, float oyf,
+                                               float ozf, RayStage* st) {
+    const double ox = oxf, oy = oyf, oz = ozf;
+    const double par0 = (ox * a.x + oy * a.y + oz * a.z) * inv;
+    const double sc = par0 * inv;
+    const double px = ox - sc * a.x, py = oy - sc * a.y, pz = oz - sc * a.z;
+    st->v[0] = (float)px; st->v[1] = (float)py; st->v[2] = (float)pz;
+    st->v[3] = u.x; st->v[4] = u.y; st->v[5] = u.z;
+}
+
+// Also true when the ray is near.
+__device__ __forceinline__ bool stage_general(const float4& a, const double4& cd, const float4& u, float oxf,
+                                              float oyf, float ozf, float hres, float rls2, RayStage* st) {
+    const double ox = oxf, oy = oyf, oz = ozf;
     const double par0 = (ox * a.x + oy * a.y + oz * a.z) * cd.z;
     const double sc = par0 * cd.z;
     const double px = ox - sc * a.x, py = oy - sc * a.y, pz = oz - sc * a.z;
-    const float ux = (float)(a.x * cd.z), uy = (float)(a.y * cd.z), uz = (float)(a.z * cd.z);
-    // centroid = anchor - res/2 on each axis; its perpendicular offset q and its distance qal
-    // along the ray beyond [0, d_m], in FP32
-    const float qd = -hres * (ux + uy + uz);
-    const float qpar = (float)par0 + qd;
-    const float qx = (float)px - hres - qd * ux, qy = (float)py - hres - qd * uy, qz = (float)pz - hres - qd * uz;
-    const float qal = fminf(qpar, 0.0f) + fmaxf(qpar - a.w, 0.0f);
-    const bool hit = box_reaches(fmaf(qal, ux, qx), fmaf(qal, uy, qy), fmaf(qal, uz, qz),
-                                 qx * qx + qy * qy + qz * qz + qal * qal, hres, rls2);
-    *near = false;
-    if (hit) {
-        const float ex = (float)(ox - a.x), ey = (float)(oy - a.y), ez = (float)(oz - a.z);
-        const float cx = ex - hres, cy = ey - hres, cz = ez - hres;
-        st[0] = make_float4((float)px, (float)py, (float)pz, (float)par0);
-        st[1] = make_float4(ux, uy, uz, (float)(par0 - cd.y));
-        st[2] = make_float4(ex, ey, ez, (float)(par0 - cd.x));
-        *near = box_reaches(cx, cy, cz, cx * cx + cy * cy + cz * cz, hres, rls2);
-    }
-    return hit;
+    const float ex = __fsub_rn(oxf, a.x), ey = __fsub_rn(oyf, a.y), ez = __fsub_rn(ozf, a.z);
+    st->v[0] = (float)px; st->v[1] = (float)py; st->v[2] = (float)pz;
+    st->v[3] = u.x; st->v[4] = u.y; st->v[5] = u.z;
+    st->v[6] = (float)par0; st->v[7] = (float)(par0 - cd.y);
+    st->v[8] = ex; st->v[9] = ey; st->v[10] = ez;
+    st->v[11] = (float)(par0 - cd.x);
+    const float cx = ex - hres, cy = ey - hres, cz = ez - hres;
+    return box_reaches(cx, cy, cz, cx * cx + cy * cy + cz * cz, hres, rls2);
 }
 
 // Two FP32 values in one 8-byte register pair for the packed f32x2 instructions of sm_100a: one
@@ -1111,24 +1201,67 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
     return d;
 }
 
-// Squared distances from the cell at offset (dx, dy, dz) from the anchor to the free segments
-// [0, margin u] of the two rays of a pair record (float4 0-3); *dpar = delta.u for each:
-// dp = delta.u, q = p + delta - dp u, al = min(par0 + dp, 0) + max(par0 - margin + dp, 0),
-// d^2 = |q|^2 + al^2.
-__device__ __forceinline__ F2 free_d2x2(const float4& b0, const float4& b1, const float4& b2, const float4& b3,
-                                        F2 DX, F2 DY, F2 DZ, F2* dpar) {
-    const F2 ux = F2::of(b2.x, b2.y), uy = F2::of(b2.z, b2.w), uz = F2::of(b3.x, b3.y);
-    const F2 dp = fma2(DZ, uz, fma2(DY, uy, mul2(DX, ux)));
-    const F2 ndp = mul2(dp, F2::of(-1.0f, -1.0f));  // exact
-    const F2 qx = fma2(ndp, ux, add2(F2::of(b0.x, b0.y), DX));
-    const F2 qy = fma2(ndp, uy, add2(F2::of(b0.z, b0.w), DY));
-    const F2 qz = fma2(ndp, uz, add2(F2::of(b1.x, b1.y), DZ));
+// A lane evaluates four cells of the sub-block, x = lane & 3, y = 2 * ((lane >> 2) & 1) + {0, 1} at
+// both heights, for one of the four pair records of a step (its quarter-warp's): a record's 8-byte
+// operands are loaded for 8 lanes x 4 cells instead of 32 lanes x 1, which divides the shared-memory
+// traffic per evaluation by four, and the parts of the arithmetic that depend on x, y or z alone are
+// done once per column. The anchor is a cell centre of the upper layer, so the upper cells' own z
+// offset is exactly 0.
+//
+// What bounds k_bgki: with one cell per lane the record loads (512 bytes returned to registers per
+// 16-byte broadcast) and the table's gathers filled half of the L1 data path each while instruction
+// issue sat at 72 %, so cutting instructions alone changed little. 256x256x32 voxels at 0.1 m,
+// 120,000 rays, 3.0e8 evaluations, evidence stage: one cell per lane, a conversion instruction per
+// value and a batch per 32 listed rays 1.51 ms; the units' sums by additions, the interior class and
+// full batches 1.38 ms; two cells per lane 1.24 ms; four 1.20 ms (200x200x25 voxels at 0.2 m, 60,000
+// rays, ls 0.5 m: 0.54 -> 0.42 ms). The warp instructions per evaluation went from 4.2 to 3.2; what
+// is left is the table's gathers (half of the L1 data path) and the waits on them. Slower here: the
+// table in shared memory (1.38 ms), predicated fetches for all cells at once (spills at 64 registers,
+// and 1.36 ms at 128 registers with 2 CTAs per SM), 3 CTAs per SM at 80 registers (1.21 ms).
+struct Cols {
+    F2 EX, EY[2], EZ;  // anchor minus the cell centres: x, both y, z of the lower cells
+    F2 TS;             // table scale
+    float ls2[4];      // ls^2 of cell (y, z) = (i & 1, i >> 1), -1 outside the grid
+};
+
+// Squared perpendicular distances of the four cells to the lines of the two rays of a pair record
+// (float4 0-2); nd = -delta.u: q = p + delta - dp u = (p - E) + nd u, squares summed in x, y, z
+// order.
+struct Perp {
+    F2 nd[4], d2[4];
+};
+__device__ __forceinline__ Perp perp_d2(const float4* __restrict__ R, const Cols& C) {
+    const float4 b0 = R[0], b1 = R[1], b2 = R[2];
+    const F2 ux = F2::of(b1.z, b1.w), uy = F2::of(b2.x, b2.y), uz = F2::of(b2.z, b2.w);
+    const F2 sx = mul2(C.EX, ux);
+    const F2 ax = sub2(F2::of(b0.x, b0.y), C.EX), py = F2::of(b0.z, b0.w), pz = F2::of(b1.x, b1.y);
+    const F2 azl = sub2(pz, C.EZ);
+    Perp r;
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+        const F2 up = fma2(C.EY[y], uy, sx), lo = fma2(C.EZ, uz, up);
+        const F2 ay = sub2(py, C.EY[y]);
+        r.nd[y] = lo;
+        r.nd[2 + y] = up;
+        {
+            const F2 qx = fma2(lo, ux, ax), qy = fma2(lo, uy, ay), qz = fma2(lo, uz, azl);
+            r.d2[y] = fma2(qz, qz, fma2(qy, qy, mul2(qx, qx)));
+        }
+        {
+            const F2 qx = fma2(up, ux, ax), qy = fma2(up, uy, ay), qz = fma2(up, uz, pz);
+            r.d2[2 + y] = fma2(qz, qz, fma2(qy, qy, mul2(qx, qx)));
+        }
+    }
+    return r;
+}
+
+// The along-ray part added to it: al = min(par0 + dp, 0) + max(par0 - margin + dp, 0).
+__device__ __forceinline__ F2 along_d2(F2 perp2, const float4& b3, F2 nd) {
     float a0, a1, e0, e1;
-    add2(F2::of(b1.z, b1.w), dp).split(a0, a1);  // d_proj
-    add2(F2::of(b3.z, b3.w), dp).split(e0, e1);  // d_proj - margin
+    sub2(F2::of(b3.x, b3.y), nd).split(a0, a1);  // d_proj
+    sub2(F2::of(b3.z, b3.w), nd).split(e0, e1);  // d_proj - margin
     const F2 al = add2(F2::of(fminf(a0, 0.0f), fminf(a1, 0.0f)), F2::of(fmaxf(e0, 0.0f), fmaxf(e1, 0.0f)));
-    *dpar = dp;
-    return fma2(al, al, fma2(qz, qz, fma2(qy, qy, mul2(qx, qx))));
+    return fma2(al, al, perp2);
 }
 
 // tab_pos for two squared distances: t = d^2 * tscale, then the floor without conversions.
@@ -1149,181 +1282,383 @@ __device__ __forceinline__ TabPos2 tab_pos2(F2 d2, F2 tscale) {
     return q;
 }
 
-// Writes the three staged float4 of a passing ray into half (slot & 1) of pair record slot / 2.
-__device__ __forceinline__ void stage_put(float* stg, int slot, const float4 st[3]) {
-    float* d = stg + (slot >> 1) * kStagePairFloats + (slot & 1);
-    d[0] = st[0].x; d[2] = st[0].y; d[4] = st[0].z; d[6] = st[0].w;
-    d[8] = st[1].x; d[10] = st[1].y; d[12] = st[1].z; d[14] = st[1].w;
-    d[16] = st[2].x; d[18] = st[2].y; d[20] = st[2].z; d[22] = st[2].w;
+// Exact sums of values in [-1, 2) in units of 2^-kFxShift, without conversion instructions. A value
+// v is split as h + l, h the nearest multiple of 2^-21 (v + 6 has that ulp) and l the exact rest;
+// l + 1.5 * 2^-17 has an ulp of one unit, so it rounds l (and with it v, since h is a multiple of
+// two units) to the nearest integer number of units, ties to even: the integer __float2ll_rn gives
+// for v * 2^40. The mantissas of the two sums are those integers plus a constant, so their bit
+// patterns are added as 32-bit integers and the constants leave once, by the number of values n.
+// Two values cost four packed additions and two three-operand integer adds; the conversion
+// instruction they replace issues at a quarter of that rate or less.
+constexpr float kFxHi = 6.0f;                    // [4, 8): ulp 2^-21
+constexpr float kFxLo = 1.5f / (1 << 17);        // [2^-17, 2^-16): ulp 2^-40
+constexpr uint32_t kFxHiBits = 0x40C00000u, kFxLoBits = 0x37400000u;
+
+struct FxSum {
+    uint32_t hi, lo;
+    __device__ __forceinline__ void add(F2 v) {
+        const F2 H = F2::of(kFxHi, kFxHi), L = F2::of(kFxLo, kFxLo);
+        const F2 t = add2(v, H);
+        const F2 q = add2(sub2(v, sub2(t, H)), L);
+        float ta, tb, qa, qb;
+        t.split(ta, tb);
+        q.split(qa, qb);
+        hi += __float_as_uint(ta) + __float_as_uint(tb);
+        lo += __float_as_uint(qa) + __float_as_uint(qb);
+    }
+    // The sum of n added values, in units; at most 2,047 values in [0, 1] (total), or 1,023 in
+    // [-1, 1] (total_signed), and kChunk plus a pad is fewer.
+    __device__ __forceinline__ long long total(uint32_t n) const {
+        return ((long long)(uint32_t)(hi - n * kFxHiBits) << 19) + (int32_t)(lo - n * kFxLoBits);
+    }
+    __device__ __forceinline__ long long total_signed(uint32_t n) const {
+        return ((long long)(int32_t)(hi - n * kFxHiBits) << 19) + (int32_t)(lo - n * kFxLoBits);
+    }
+};
+
+// Writes the first N staged constants of a candidate into half (slot & 1) of pair record slot / 2.
+template <int REC, int N>
+__device__ __forceinline__ void stage_put(float* stg, int slot, const RayStage& st) {
+    float* d = stg + (slot >> 1) * REC + (slot & 1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) d[2 * i] = st.v[i];
 }
 
-// A pad ray in slot (odd, < 32): perpendicular and point offsets of 1e15 put every cell at a
-// squared distance near 3e30 (finite in FP32, far beyond ls^2), and d_proj - d_m = d_proj = 0
-// fails the d_proj < d_m test, so the pad adds nothing.
-__device__ __forceinline__ void stage_pad(float* stg, int slot) {
-    const float4 big = make_float4(1e15f, 1e15f, 1e15f, 0.0f);
-    const float4 st[3] = {big, make_float4(0.0f, 0.0f, 0.0f, 0.0f), big};
-    stage_put(stg, slot, st);
+// A pad ray: perpendicular and point offsets of 1e15 put every cell at a squared distance near 3e30
+// (finite in FP32, far beyond ls^2), and d_proj - d_m = d_proj = 0 fails the d_proj < d_m test, so
+// the pad adds nothing.
+__device__ __forceinline__ RayStage pad_ray() {
+    RayStage st;
+#pragma unroll
+    for (int i = 0; i < 12; ++i) st.v[i] = (i < 3 || (i >= 8 && i < 11)) ? 1e15f : 0.0f;
+    return st;
 }
 
-template <int MINB, int THREADS = kEvThreads, bool REGIONS = false>
-__global__ void __launch_bounds__(THREADS, MINB) k_bgki(EvArgs A) {
-    extern __shared__ __align__(32) unsigned char smem_raw[];
-    const BgkiSmem S = bgki_smem(smem_raw, A.chunk, THREADS / 32);
-    __shared__ uint32_t s_item;
-    __shared__ int s_next_sb, s_last;
+// Batches of up to 32 candidate rays (r of each lane; the first n lanes hold one) against the
+// sub-block with anchor (ox, oy, oz): FP64 resolution, pair records (padded to a multiple of four
+// records by rays that reach no cell), evaluation. V evaluates: occ(i, pos, a, b) and free(...) take
+// the table positions of a pair and whether each ray's value counts for the lane's cell i.
+template <class V>
+__device__ __forceinline__ void interior_batch(const EvArgs& A, const BgkiSmem& S, const Cols& C, float ox, float oy,
+                                               float oz, float* stg, int r, int n, V& ev) {
+    const int lane = threadIdx.x & 31;
+    {
+        RayStage st = pad_ray();
+        if (lane < n) {
+            const uint32_t rid = S.rid[r];
+            stage_interior(__ldg(A.ray_a + rid), __ldg(&A.ray_c[rid].z), S.u[r], ox, oy, oz, &st);
+        }
+        stage_put<kRecInterior, 6>(stg, lane, st);
+        __syncwarp();
+    }
+    const int steps = (n + 7) >> 3;
+    const float* rec = stg + (lane >> 3) * kRecInterior;  // the quarter-warp's record of each step
+#pragma unroll 1
+    for (int k = 0; k < steps; ++k, rec += 4 * kRecInterior) {
+        const Perp p = perp_d2(reinterpret_cast<const float4*>(rec), C);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float da, db;
+            p.d2[i].split(da, db);
+            ev.free(i, tab_pos2(p.d2[i], C.TS), da < C.ls2[i], db < C.ls2[i]);
+        }
+    }
+    ev.n_free += steps;
+    __syncwarp();
+}
+
+template <class V>
+__device__ __forceinline__ void general_batch(const EvArgs& A, const BgkiSmem& S, const ItemConst& I, const Cols& C,
+                                              float ox, float oy, float oz, float* stg, int r, int n, V& ev) {
+    const int lane = threadIdx.x & 31;
+    int near_steps;
+    {
+        RayStage st = pad_ray();
+        bool near = false;
+        if (lane < n) {
+            const uint32_t rid = S.rid[r];
+            const double2* c = reinterpret_cast<const double2*>(A.ray_c + rid);
+            const double2 c0 = __ldg(c), c1 = __ldg(c + 1);
+            near = stage_general(__ldg(A.ray_a + rid), make_double4(c0.x, c0.y, c1.x, 0.0), S.u[r], ox, oy, oz,
+                                 0.5f * I.res, I.rls2, &st);
+        }
+        // near rays first; a step that holds one evaluates all its rays as near, which adds nothing
+        // for the others
+        const unsigned m = __ballot_sync(0xffffffffu, near);
+        const int nn = __popc(m), below = __popc(m & ((1u << lane) - 1u));
+        stage_put<kRecGeneral, 12>(stg, near ? below : nn + lane - below, st);
+        near_steps = (nn + 7) >> 3;
+        __syncwarp();
+    }
+    const int steps = (n + 7) >> 3;
+    const float* rec = stg + (lane >> 3) * kRecGeneral;
+    int k = 0;
+    // steps holding a near ray: occupied (mass_update.cu:48-52) and free (:54-71) evidence
+    ev.begin_occ();
+#pragma unroll 1
+    for (; k < near_steps; ++k, rec += 4 * kRecGeneral) {
+        const float4* R = reinterpret_cast<const float4*>(rec);
+        float da, db;
+        {
+            const float4 b4 = R[4], b5 = R[5];
+            const F2 vx = sub2(F2::of(b4.x, b4.y), C.EX), vz = F2::of(b5.x, b5.y), vl = sub2(vz, C.EZ);
+            const F2 xx = mul2(vx, vx);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const F2 vy = sub2(F2::of(b4.z, b4.w), C.EY[i & 1]);
+                const F2 w = i < 2 ? vl : vz;
+                const F2 d2 = fma2(w, w, fma2(vy, vy, xx));
+                d2.split(da, db);
+                ev.occ(i, tab_pos2(d2, C.TS), da < C.ls2[i], db < C.ls2[i]);
+            }
+        }
+        const Perp p = perp_d2(R, C);
+        const float4 b3 = R[3], b5 = R[5];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const F2 d2 = along_d2(p.d2[i], b3, p.nd[i]);
+            float ea, eb;
+            d2.split(da, db);
+            sub2(F2::of(b5.z, b5.w), p.nd[i]).split(ea, eb);  // d_proj - d_m
+            ev.free(i, tab_pos2(d2, C.TS), ea < 0.0f && da < C.ls2[i], eb < 0.0f && db < C.ls2[i]);
+        }
+    }
+    if (near_steps) ev.end_occ(near_steps);
+    // the other steps: free evidence only
+#pragma unroll 1
+    for (; k < steps; ++k, rec += 4 * kRecGeneral) {
+        const float4* R = reinterpret_cast<const float4*>(rec);
+        const Perp p = perp_d2(R, C);
+        const float4 b3 = R[3];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const F2 d2 = along_d2(p.d2[i], b3, p.nd[i]);
+            float da, db;
+            d2.split(da, db);
+            ev.free(i, tab_pos2(d2, C.TS), da < C.ls2[i], db < C.ls2[i]);
+        }
+    }
+    ev.n_free += steps;
+    __syncwarp();
+}
+
+// The evidence of sub-block sb of the item: the cull of its listed rays (its region's, or all of
+// the item's), their batches, and the cells' sums.
+template <class V>
+__device__ __forceinline__ void eval_sub_block(const EvArgs& A, const BgkiSmem& S, const ItemConst& I, int sb,
+                                               const int* rcnt, float* stg, uint16_t* ring, V& ev) {
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const uint16_t* list = nullptr;
+    int nlist = I.nr;
+    if (I.regions) {
+        const int q = sb_region(I.ts, sb);
+        list = S.reg + q * A.chunk;
+        nlist = rcnt[q];
+    }
+    if (nlist == 0) return;
+    Cols C;
+    float ox, oy, oz;
+    {
+        DevParams p;  // the fields centre_xyz reads
+        p.G = I.G; p.Gz = I.Gz; p.res = I.res;
+        const SbCell b = sb_cell(I.ts, I.lt, sb);
+        const int ix = b.x + (lane & 3), iy = b.y + 2 * ((lane >> 2) & 1);
+        float x, y0, y1, z, t;
+        centre_xyz(ix, iy, b.z, p, I.sx, I.sy, I.sz, &x, &y0, &z);
+        centre_xyz(ix, iy + 1, b.z, p, I.sx, I.sy, I.sz, &t, &y1, &t);
+        centre_xyz(b.x + 2, b.y + 2, b.z + 1, p, I.sx, I.sy, I.sz, &ox, &oy, &oz);
+        // exact (nearby floats)
+        const float ex = ox - x, ey0 = oy - y0, ey1 = oy - y1, ez = oz - z, ts = I.tscale;
+        C.EX = F2::of(ex, ex); C.EY[0] = F2::of(ey0, ey0); C.EY[1] = F2::of(ey1, ey1); C.EZ = F2::of(ez, ez);
+        C.TS = F2::of(ts, ts);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            C.ls2[i] = ix < I.G && iy + (i & 1) < I.G && b.z + (i >> 1) < I.Gz ? I.ls2 : -1.0f;
+    }
+    ev.begin(I);
+    uint16_t* gring = ring + kRing;
+    int head = 0, n = 0, ghead = 0, gn = 0;  // interior and general candidates
+    for (int g0 = 0; g0 < nlist; g0 += 32) {
+        const int j = g0 + lane;
+        int r = j;
+        RayClass cls = kRayNone;
+        if (j < nlist) {
+            if (list) r = list[j];
+            const float hres = 0.5f * I.res;
+            const float cx = ox - hres, cy = oy - hres, cz = oz - hres;
+            const float eps = 1e-6f * (fabsf(cx) + fabsf(cy) + fabsf(cz));
+            cls = cull_ray(S.u[r], cx, cy, cz, hres, I.rls + eps, eps);
+        }
+        const unsigned mi = __ballot_sync(0xffffffffu, cls == kRayInterior);
+        const unsigned mg = __ballot_sync(0xffffffffu, cls == kRayGeneral);
+        if (cls == kRayInterior) ring[(head + n + __popc(mi & below)) & (kRing - 1)] = (uint16_t)r;
+        if (cls == kRayGeneral) gring[(ghead + gn + __popc(mg & below)) & (kRing - 1)] = (uint16_t)r;
+        n += __popc(mi);
+        gn += __popc(mg);
+        const bool last = g0 + 32 >= nlist;
+        if (n < 32 && gn < 32 && !last) continue;
+        __syncwarp();
+        // full batches, and what is left after the last group
+#pragma unroll 1
+        for (; n >= 32 || (last && n > 0); n -= 32, head += 32)
+            interior_batch(A, S, C, ox, oy, oz, stg, ring[(head + lane) & (kRing - 1)], min(n, 32), ev);
+#pragma unroll 1
+        for (; gn >= 32 || (last && gn > 0); gn -= 32, ghead += 32)
+            general_batch(A, S, I, C, ox, oy, oz, stg, gring[(ghead + lane) & (kRing - 1)], min(gn, 32), ev);
+    }
+    // lane's output cell: column (lane & 7) of its four cells, the one of its quarter-warp
+    const SbCell b = sb_cell(I.ts, I.lt, sb);
+    const int q = lane >> 3;
+    const int ix = b.x + (lane & 3), iy = b.y + 2 * ((lane >> 2) & 1) + (q & 1), iz = b.z + (q >> 1);
+    const bool in = ix < I.G && iy < I.G && iz < I.Gz;
+    ev.end(A, (long)I.coff + ix + I.G * iy + I.G * I.G * iz, in);
+}
+
+// The four quarter-warps' sums of the lane's four cells, added up: quarter q keeps cell q.
+__device__ __forceinline__ FxSum quarter_merge(const FxSum s[4]) {
+    const bool odd = (threadIdx.x & 8) != 0, up = (threadIdx.x & 16) != 0;
+    FxSum k[2];  // cells (odd, z = 0, 1) of two quarters
+#pragma unroll
+    for (int z = 0; z < 2; ++z) {
+        const FxSum mine = odd ? s[2 * z + 1] : s[2 * z], other = odd ? s[2 * z] : s[2 * z + 1];
+        k[z].hi = mine.hi + __shfl_xor_sync(0xffffffffu, other.hi, 8);
+        k[z].lo = mine.lo + __shfl_xor_sync(0xffffffffu, other.lo, 8);
+    }
+    const FxSum mine = up ? k[1] : k[0], other = up ? k[0] : k[1];
+    return FxSum{mine.hi + __shfl_xor_sync(0xffffffffu, other.hi, 16),
+                 mine.lo + __shfl_xor_sync(0xffffffffu, other.lo, 16)};
+}
+
+// K3DOM values: the scene's table through the texture path. FMA.SAT turns a negative table value
+// (the kernel's max(0, .)) into 0; values are at most 1. The free sums are kept for the lane's four
+// cells, the occupied ones (few rays are near) are merged after every run of near steps.
+struct K3domEval {
+    cudaTextureObject_t tex;
+    int base;                   // the scene's table in the texture
+    FxSum so[4], sf[4], occ_sum;
+    int n_occ, n_free;          // steps added (two values per quarter-warp and step)
+    unsigned nev;               // in-support evaluations of this lane (the roofline's work count)
+    __device__ __forceinline__ void begin(const ItemConst& I) {
+        base = I.tbase;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sf[i] = FxSum{0u, 0u};
+        occ_sum = FxSum{0u, 0u};
+        n_occ = n_free = 0;
+    }
+    __device__ __forceinline__ void begin_occ() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) so[i] = FxSum{0u, 0u};
+    }
+    __device__ __forceinline__ void end_occ(int steps) {
+        const FxSum o = quarter_merge(so);
+        occ_sum.hi += o.hi;
+        occ_sum.lo += o.lo;
+        n_occ += steps;
+    }
+    __device__ __forceinline__ float value(const TabPos& q) {
+        const float4 c = tex1Dfetch<float4>(tex, base + q.i);
+        return __saturatef(fmaf(q.f, fmaf(q.f, fmaf(q.f, c.w, c.z), c.y), c.x));
+    }
+    __device__ __forceinline__ F2 pair(const TabPos2& q, bool a, bool b) {
+        float va = 0.0f, vb = 0.0f;
+        if (a) { va = value(q.a); ++nev; }
+        if (b) { vb = value(q.b); ++nev; }
+        return F2::of(va, vb);
+    }
+    __device__ __forceinline__ void occ(int i, const TabPos2& q, bool a, bool b) { so[i].add(pair(q, a, b)); }
+    __device__ __forceinline__ void free(int i, const TabPos2& q, bool a, bool b) { sf[i].add(pair(q, a, b)); }
+    __device__ __forceinline__ void end(const EvArgs& A, long c, bool in) {
+        const FxSum f = quarter_merge(sf);
+        if (!in) return;
+        unsigned long long* ac = A.acc + 2 * c;
+        const long long vo = occ_sum.total(8u * n_occ), vf = f.total(8u * n_free);
+        if (vo) atomicAdd(ac, (unsigned long long)vo);
+        if (vf) atomicAdd(ac + 1, (unsigned long long)vf);
+    }
+};
+
+// The work loop of a persistent CTA: items from the device counter, each staged by the whole CTA,
+// its sub-blocks pulled by the warps; done(I) runs on every thread after an item's last sub-block
+// (between barriers).
+template <class V, class D>
+__device__ __forceinline__ void run_items(const EvArgs& A, unsigned char* smem, V& ev, D done) {
+    __shared__ ItemConst I;
+    __shared__ int s_next_sb;
     __shared__ SbOrder s_order;
     __shared__ int s_rcnt[kRegions];
+    const BgkiSmem S = bgki_smem(smem, A.chunk);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned lanes_below = (1u << lane) - 1u;
-    const Batch& bt = A.bt;
-    const uint32_t total_items = A.item_off[bt.T];
-    unsigned nev = 0;      // in-support evaluations of this lane (the roofline's work count)
-
+    const uint32_t total_items = A.item_off[A.bt.T];
     for (;;) {
-        if (threadIdx.x == 0) {
-            s_item = atomicAdd(&A.status->work_counter, 1u);
-            s_next_sb = 0;
+        if (wid == 0) fetch_item(A, total_items, A.chunk, &I);
+        if (threadIdx.x < kRegions) s_rcnt[threadIdx.x] = 0;
+        if (threadIdx.x == kEvThreads - 1) s_next_sb = 0;
+        __syncthreads();
+        if (!I.live) break;
+        stage_item_rays(A, I, S, s_rcnt);
+        {
+            DevParams p;
+            p.G = I.G; p.Gz = I.Gz; p.res = I.res;
+            sb_order_keys(s_order, p, I.ts, I.lt, I.nsb, I.sx, I.sy, I.sz);
         }
-        if (REGIONS && threadIdx.x < kRegions) s_rcnt[threadIdx.x] = 0;
         __syncthreads();
-        const uint32_t item = s_item;
-        if (item >= total_items) break;
-        const Item it = item_of(bt, A.item_off, A.tile_start, item, A.chunk);
-        const SceneDev& sd = bt.sc[it.sc];
-        const DevParams& p = sd.p;
-        const TileShape ts = sd.ts;
-        const FrameParams fp = bt.fp[it.sc];
-        const int coff = bt.off->cell[it.sc];
-        const float ls2 = p.ls * p.ls;
-        const float tscale = (1.0f / ls2) * (float)kKernelTab;  // d^2 -> table position
-        const float hres = 0.5f * p.res;
-        const float cull_ls2 = sd.cull_ls2;
-        const int nsb = ts.nsbx * ts.nsby * (ts.tz / 2);
-        const int tbase = it.sc * kKernelTabEntries;  // the scene's table in the texture
-        const bool regions = REGIONS && ts.tx == 16 && ts.ty == 16;
-        stage_item_rays<THREADS>(A, it, sd, fp, regions, S.a, S.c, S.reg, s_rcnt);
-        sb_order_keys(s_order, p, ts, it.lt, nsb, fp.sensor_x, fp.sensor_y, fp.sensor_z);
+        sb_order_rank(s_order, I.nsb);
         __syncthreads();
-        sb_order_rank(s_order, nsb);
-        __syncthreads();
-        const int nr = it.nr;
         for (;;) {
             int sb = 0;
             if (lane == 0) sb = atomicAdd(&s_next_sb, 1);
             sb = __shfl_sync(0xffffffffu, sb, 0);
-            if (sb >= nsb) break;
-            sb = sb_at(s_order, sb, nsb);
-            const CellLoc L = locate(p, ts, it.lt, sb, lane, fp.sensor_x, fp.sensor_y, fp.sensor_z);
-            const float dx = L.x - L.ox, dy = L.y - L.oy, dz = L.z - L.oz;  // exact (nearby floats)
-            const float ls2c = L.c >= 0 ? ls2 : -1.0f;  // cells outside the grid take no evidence
-            const double ox = L.ox, oy = L.oy, oz = L.oz;
-            const F2 DX = F2::of(dx, dx), DY = F2::of(dy, dy), DZ = F2::of(dz, dz), TS = F2::of(tscale, tscale);
-            float* stg = S.stage + wid * kStageWarpFloats;
-            // sums of kernel values rounded to integer units; the unsigned conversion saturates a
-            // negative table value (the kernel's max(0, .)) to 0
-            unsigned long long ao = 0, af = 0;
-            // the rays to cull: the sub-block's region list, or every ray of the item
-            const int q = sb_region(ts, sb);
-            const int nlist = regions ? s_rcnt[q] : nr;
-            const uint16_t* list = S.reg + q * A.chunk;
-            for (int g0 = 0; g0 < nlist; g0 += 32) {
-                const int j = g0 + lane;
-                bool hit = false, near = false;
-                float4 st[3];
-                if (j < nlist) {
-                    const int r = regions ? (int)list[j] : j;
-                    hit = stage_pair(S.a[r], S.c[r], ox, oy, oz, hres, cull_ls2, st, &near);
-                }
-                // compact the passing rays into the warp's staging list, near rays first, two rays
-                // to a pair record; an odd count ends in a pad ray that reaches no cell
-                const unsigned mnear = __ballot_sync(0xffffffffu, near);
-                const unsigned mfar = __ballot_sync(0xffffffffu, hit && !near);
-                const int nn = __popc(mnear), nh = nn + __popc(mfar);
-                if (hit) stage_put(stg, near ? __popc(mnear & lanes_below) : nn + __popc(mfar & lanes_below), st);
-                if ((nh & 1) && lane == 0) stage_pad(stg, nh);
-                __syncwarp();
-                // pairs holding a ray whose point's sphere can reach the sub-block: occupied
-                // (mass_update.cu:48-52) and free (:54-71) evidence; a far ray sharing such a pair
-                // adds nothing through the occupied term or the d_proj < d_m test (see stage_pair)
-                const int npn = (nn + 1) >> 1, npa = (nh + 1) >> 1;
-                for (int k = 0; k < npn; ++k) {
-                    const float4* B = reinterpret_cast<const float4*>(stg + k * kStagePairFloats);
-                    {  // occupied term
-                        const float4 b4 = B[4], b5 = B[5];
-                        const F2 vx = add2(F2::of(b4.x, b4.y), DX), vy = add2(F2::of(b4.z, b4.w), DY);
-                        const F2 vz = add2(F2::of(b5.x, b5.y), DZ);
-                        const F2 d2o = fma2(vz, vz, fma2(vy, vy, mul2(vx, vx)));
-                        float oa, ob;
-                        d2o.split(oa, ob);
-                        const TabPos2 po = tab_pos2(d2o, TS);
-                        if (oa < ls2c) { ao += __float2ull_rn(tab_eval_tex(A.ktex, tbase, po.a)); ++nev; }
-                        if (ob < ls2c) { ao += __float2ull_rn(tab_eval_tex(A.ktex, tbase, po.b)); ++nev; }
-                    }
-                    F2 dp;
-                    const F2 d2f = free_d2x2(B[0], B[1], B[2], B[3], DX, DY, DZ, &dp);
-                    const float4 b5 = B[5];
-                    const F2 toend = add2(F2::of(b5.z, b5.w), dp);  // d_proj - d_m
-                    float fa, fb, ea, eb;
-                    d2f.split(fa, fb);
-                    toend.split(ea, eb);
-                    const TabPos2 pf = tab_pos2(d2f, TS);
-                    if (ea < 0.0f && fa < ls2c) { af += __float2ull_rn(tab_eval_tex(A.ktex, tbase, pf.a)); ++nev; }
-                    if (eb < 0.0f && fb < ls2c) { af += __float2ull_rn(tab_eval_tex(A.ktex, tbase, pf.b)); ++nev; }
-                }
-                // the other pairs: free evidence only
-                for (int k = npn; k < npa; ++k) {
-                    const float4* B = reinterpret_cast<const float4*>(stg + k * kStagePairFloats);
-                    F2 dp;
-                    const F2 d2f = free_d2x2(B[0], B[1], B[2], B[3], DX, DY, DZ, &dp);
-                    float fa, fb;
-                    d2f.split(fa, fb);
-                    const TabPos2 pf = tab_pos2(d2f, TS);
-                    if (fa < ls2c) { af += __float2ull_rn(tab_eval_tex(A.ktex, tbase, pf.a)); ++nev; }
-                    if (fb < ls2c) { af += __float2ull_rn(tab_eval_tex(A.ktex, tbase, pf.b)); ++nev; }
-                }
-                __syncwarp();
-            }
-            if (L.c >= 0) {
-                unsigned long long* ac = A.acc + 2 * (long)(coff + L.c);
-                if (ao) atomicAdd(ac, ao);
-                if (af) atomicAdd(ac + 1, af);
-            }
+            if (sb >= I.nsb) break;
+            eval_sub_block(A, S, I, sb_at(s_order, sb, I.nsb), s_rcnt, S.stage + wid * kStageWarpFloats,
+                           S.ring + 2 * wid * kRing, ev);
         }
-        if (!A.fuse_update) {  // the cells are updated by k_k3dom_update_cells after this kernel
-            __syncthreads();
-            continue;
-        }
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) s_last = (atomicAdd(&A.tile_done[it.t], 1u) == it.n_items - 1) ? 1 : 0;
-        __syncthreads();
-        if (s_last) {
-            __threadfence();
-            const int tx = it.lt % ts.ntx, ty = (it.lt / ts.ntx) % ts.nty, tz = it.lt / (ts.ntx * ts.nty);
-            const int tile_cells = ts.tx * ts.ty * ts.tz;
-            for (int li = threadIdx.x; li < tile_cells; li += THREADS) {
-                const int lx = li % ts.tx, ly = (li / ts.tx) % ts.ty, lz = li / (ts.tx * ts.ty);
-                const int ix = tx * ts.tx + lx, iy = ty * ts.ty + ly, iz = tz * ts.tz + lz;
-                if (ix >= p.G || iy >= p.G || iz >= p.Gz) continue;
-                const int c = coff + ix + p.G * iy + p.G * p.G * iz;
-                // every chunk of the tile has added its share (fence + tile counter above); read
-                // the totals from L2 and clear only what was written
-                unsigned long long* ac = A.acc + 2 * (long)c;
-                const long long fo = (long long)__ldcg(ac);
-                const long long ff = (long long)__ldcg(ac + 1);
-                if (fo) __stcg(ac, 0ull);
-                if (ff) __stcg(ac + 1, 0ull);
-                k3dom_cell_update(p, fp.gamma_dt, c, (double)fo * sd.fx_inv, (double)ff * sd.fx_inv, A.cs, A.cw,
-                                  A.first_frame != 0);
-            }
-            if (threadIdx.x == 0) A.tile_done[it.t] = 0;
-        }
+        done(I);
         __syncthreads();
     }
+}
+
+__global__ void __launch_bounds__(kEvThreads, kEvCtas) k_bgki(EvArgs A) {
+    extern __shared__ __align__(32) unsigned char smem_raw[];
+    __shared__ int s_last;
+    K3domEval ev;
+    ev.tex = A.ktex;
+    ev.nev = 0;
+    run_items(A, smem_raw, ev, [&](const ItemConst& I) {
+        if (!A.fuse_update) return;  // the cells are updated by k_k3dom_update_cells after this kernel
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = (atomicAdd(&A.tile_done[I.t], 1u) == I.n_items - 1) ? 1 : 0;
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        const SceneDev& sd = A.bt.sc[I.sc];
+        const DevParams& p = sd.p;
+        const TileShape ts = I.ts;
+        const double gdt = A.bt.fp[I.sc].gamma_dt;
+        const int tx = I.lt % ts.ntx, ty = (I.lt / ts.ntx) % ts.nty, tz = I.lt / (ts.ntx * ts.nty);
+        const int tile_cells = ts.tx * ts.ty * ts.tz;
+        for (int li = threadIdx.x; li < tile_cells; li += kEvThreads) {
+            const int lx = li % ts.tx, ly = (li / ts.tx) % ts.ty, lz = li / (ts.tx * ts.ty);
+            const int ix = tx * ts.tx + lx, iy = ty * ts.ty + ly, iz = tz * ts.tz + lz;
+            if (ix >= p.G || iy >= p.G || iz >= p.Gz) continue;
+            const int c = I.coff + ix + p.G * iy + p.G * p.G * iz;
+            // every chunk of the tile has added its share (fence + tile counter above); read
+            // the totals from L2 and clear only what was written
+            unsigned long long* ac = A.acc + 2 * (long)c;
+            const long long fo = (long long)__ldcg(ac);
+            const long long ff = (long long)__ldcg(ac + 1);
+            if (fo) __stcg(ac, 0ull);
+            if (ff) __stcg(ac + 1, 0ull);
+            k3dom_cell_update(p, gdt, c, (double)fo * sd.fx_inv, (double)ff * sd.fx_inv, A.cs, A.cw,
+                              A.first_frame != 0);
+        }
+        if (threadIdx.x == 0) A.tile_done[I.t] = 0;
+    });
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) nev += __shfl_xor_sync(0xffffffffu, nev, o);
-    if (lane == 0 && nev) atomicAdd(&A.status->kernel_evals, (unsigned long long)nev);
+    for (int o = 16; o > 0; o >>= 1) ev.nev += __shfl_xor_sync(0xffffffffu, ev.nev, o);
+    if (lane == 0 && ev.nev) atomicAdd(&A.status->kernel_evals, (unsigned long long)ev.nev);
 }
 
 // ================================================================ DS-PHD/MIB
@@ -1717,192 +2052,102 @@ static void build_table(double (*fn)(double), double scale, float4* out) {
 }
 
 void build_calib_tables(float4* f_tab, float4* dls_tab) {
-    build_table(unit_kernel, std::ldexp(1.0, kCalibShift), f_tab);
-    build_table(unit_kernel_dls, std::ldexp(1.0, kCalibShift), dls_tab);
+    build_table(unit_kernel, 1.0, f_tab);
+    build_table(unit_kernel_dls, 1.0, dls_tab);
 }
 
-// Shared memory of k_bgki_sums (dynamic, sized by the work item's ray count).
-struct CalibSmem {
-    float4* ftab;            // [kKernelTabEntries] unit kernel f, fixed-point scale folded in
-    float4* htab;            // [kKernelTabEntries] -x f'(x), same scale
-    float* stage;            // [kEvWarps][kStageWarpFloats] pair records, as in k_bgki
-    float4* a;               // [chunk]
-    double4* c;              // [chunk]
-    uint16_t* reg;           // [kRegions][chunk] (region builds)
+// The calibration's values: f and -x f' from two tables in shared memory (through the texture path
+// they measured slower), two sums per evidence kind. f is clamped at 0 by FMA.SAT, -x f' lies in
+// [-3e-7, 0.78].
+static_assert(kCalibShift == kFxShift, "units of the calibration sums");
+
+struct CalibEval {
+    const float4 *ftab, *htab;  // [kKernelTabEntries] each
+    unsigned long long* acc4;
+    FxSum fo[4], ff[4], ho[4], hf[4], occ_f, occ_h;
+    int n_occ, n_free;
+    __device__ __forceinline__ void begin(const ItemConst&) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) ff[i] = hf[i] = FxSum{0u, 0u};
+        occ_f = occ_h = FxSum{0u, 0u};
+        n_occ = n_free = 0;
+    }
+    __device__ __forceinline__ void begin_occ() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) fo[i] = ho[i] = FxSum{0u, 0u};
+    }
+    __device__ __forceinline__ void end_occ(int steps) {
+        const FxSum f = quarter_merge(fo), h = quarter_merge(ho);
+        occ_f.hi += f.hi;
+        occ_f.lo += f.lo;
+        occ_h.hi += h.hi;
+        occ_h.lo += h.lo;
+        n_occ += steps;
+    }
+    __device__ __forceinline__ void value(const TabPos& q, float* f, float* h) {
+        const float4 c = ftab[q.i], d = htab[q.i];
+        *f = __saturatef(fmaf(q.f, fmaf(q.f, fmaf(q.f, c.w, c.z), c.y), c.x));
+        *h = fmaf(q.f, fmaf(q.f, fmaf(q.f, d.w, d.z), d.y), d.x);
+    }
+    __device__ __forceinline__ void pair(const TabPos2& q, bool a, bool b, FxSum& f, FxSum& h) {
+        float fa = 0.0f, fb = 0.0f, ha = 0.0f, hb = 0.0f;
+        if (a) value(q.a, &fa, &ha);
+        if (b) value(q.b, &fb, &hb);
+        f.add(F2::of(fa, fb));
+        h.add(F2::of(ha, hb));
+    }
+    __device__ __forceinline__ void occ(int i, const TabPos2& q, bool a, bool b) { pair(q, a, b, fo[i], ho[i]); }
+    __device__ __forceinline__ void free(int i, const TabPos2& q, bool a, bool b) { pair(q, a, b, ff[i], hf[i]); }
+    __device__ __forceinline__ void end(const EvArgs&, long c, bool in) {
+        const FxSum sff = quarter_merge(ff), shf = quarter_merge(hf);
+        if (!in) return;
+        unsigned long long* ac = acc4 + 4 * c;
+        const uint32_t no = 8u * n_occ, nf = 8u * n_free;
+        const long long v[4] = {occ_f.total(no), sff.total(nf), occ_h.total_signed(no), shf.total_signed(nf)};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (v[i]) atomicAdd(ac + i, (unsigned long long)v[i]);
+    }
 };
 
-constexpr size_t kCalibFixedBytes =
-    2 * sizeof(float4) * kKernelTabEntries + sizeof(float) * (size_t)kEvWarps * kStageWarpFloats;
+constexpr size_t kCalibTabBytes = (2 * sizeof(float4) * kKernelTabEntries + 31) & ~(size_t)31;
 
-inline size_t calib_smem_bytes(int chunk, bool regions = false) {
-    return ((kCalibFixedBytes + 31) & ~(size_t)31) + (size_t)chunk * (sizeof(float4) + sizeof(double4)) +
-           (regions ? (size_t)kRegions * chunk * sizeof(uint16_t) : 0);
-}
-
-__device__ __forceinline__ CalibSmem calib_smem(unsigned char* base, int chunk) {
-    CalibSmem S;
-    S.ftab = reinterpret_cast<float4*>(base);
-    S.htab = S.ftab + kKernelTabEntries;
-    S.stage = reinterpret_cast<float*>(base + 2 * sizeof(float4) * kKernelTabEntries);
-    const size_t off = (kCalibFixedBytes + 31) & ~(size_t)31;
-    S.c = reinterpret_cast<double4*>(base + off);
-    S.a = reinterpret_cast<float4*>(base + off + sizeof(double4) * (size_t)chunk);
-    S.reg = reinterpret_cast<uint16_t*>(base + off + (sizeof(double4) + sizeof(float4)) * (size_t)chunk);
-    return S;
-}
+inline size_t calib_smem_bytes(int chunk) { return kCalibTabBytes + bgki_smem_bytes(chunk); }
 
 // acc4: 4 signed 64-bit sums per cell (f occ, f free, -x f' occ, -x f' free), in units. Same
 // tiles, culls and pair geometry as k_bgki; each value is rounded once to an integer number of
 // units (round to nearest even).
-template <int MINB, bool REGIONS = false>
-__global__ void __launch_bounds__(kEvThreads, MINB) k_bgki_sums(EvArgs A, const float4* __restrict__ htab,
+__global__ void __launch_bounds__(kEvThreads, kEvCtas) k_bgki_sums(EvArgs A, const float4* __restrict__ htab,
                                                                unsigned long long* __restrict__ acc4) {
     extern __shared__ __align__(32) unsigned char smem_raw[];
-    const CalibSmem S = calib_smem(smem_raw, A.chunk);
-    __shared__ uint32_t s_item;
-    __shared__ int s_next_sb;
-    __shared__ SbOrder s_order;
-    __shared__ int s_rcnt[kRegions];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned lanes_below = (1u << lane) - 1u;
-    const Batch& bt = A.bt;
-    const uint32_t total_items = A.item_off[bt.T];
-    for (int i = threadIdx.x; i < kKernelTabEntries; i += kEvThreads) {
-        S.ftab[i] = A.ktab[i];
-        S.htab[i] = htab[i];
+    float4* tab = reinterpret_cast<float4*>(smem_raw);
+    for (int i = threadIdx.x; i < kKernelTabEntries; i += kEvThreads) {  // used after run_items' first barrier
+        tab[i] = A.ktab[i];
+        tab[kKernelTabEntries + i] = htab[i];
     }
-    for (;;) {
-        if (threadIdx.x == 0) {
-            s_item = atomicAdd(&A.status->work_counter, 1u);
-            s_next_sb = 0;
-        }
-        if (REGIONS && threadIdx.x < kRegions) s_rcnt[threadIdx.x] = 0;
-        __syncthreads();
-        const uint32_t item = s_item;
-        if (item >= total_items) break;
-        const Item it = item_of(bt, A.item_off, A.tile_start, item, A.chunk);
-        const SceneDev& sd = bt.sc[it.sc];
-        const DevParams& p = sd.p;
-        const TileShape ts = sd.ts;
-        const FrameParams fp = bt.fp[it.sc];
-        const int coff = bt.off->cell[it.sc];
-        const float ls2 = p.ls * p.ls;
-        const float tscale = (1.0f / ls2) * (float)kKernelTab;  // d^2 -> table position
-        const float hres = 0.5f * p.res;
-        const float cull_ls2 = sd.cull_ls2;
-        const int nsb = ts.nsbx * ts.nsby * (ts.tz / 2);
-        const bool regions = REGIONS && ts.tx == 16 && ts.ty == 16;
-        stage_item_rays<kEvThreads>(A, it, sd, fp, regions, S.a, S.c, S.reg, s_rcnt);
-        sb_order_keys(s_order, p, ts, it.lt, nsb, fp.sensor_x, fp.sensor_y, fp.sensor_z);
-        __syncthreads();
-        sb_order_rank(s_order, nsb);
-        __syncthreads();
-        const int nr = it.nr;
-        for (;;) {
-            int sb = 0;
-            if (lane == 0) sb = atomicAdd(&s_next_sb, 1);
-            sb = __shfl_sync(0xffffffffu, sb, 0);
-            if (sb >= nsb) break;
-            sb = sb_at(s_order, sb, nsb);
-            const CellLoc L = locate(p, ts, it.lt, sb, lane, fp.sensor_x, fp.sensor_y, fp.sensor_z);
-            const float dx = L.x - L.ox, dy = L.y - L.oy, dz = L.z - L.oz;
-            const float ls2c = L.c >= 0 ? ls2 : -1.0f;
-            const double ox = L.ox, oy = L.oy, oz = L.oz;
-            const F2 DX = F2::of(dx, dx), DY = F2::of(dy, dy), DZ = F2::of(dz, dz), TS = F2::of(tscale, tscale);
-            float* stg = S.stage + wid * kStageWarpFloats;
-            long long fo = 0, ff = 0, ho = 0, hf = 0;
-            const int q = sb_region(ts, sb);
-            const int nlist = regions ? s_rcnt[q] : nr;
-            const uint16_t* list = S.reg + q * A.chunk;
-            // one in-support evaluation: f (clamped at 0, as the kernel is) and -x f' at position t
-            auto eval = [&](TabPos t, long long& f, long long& h) {
-                f += __float2ll_rn(fmaxf(tab_eval(S.ftab, t), 0.0f));
-                h += __float2ll_rn(tab_eval(S.htab, t));
-            };
-            for (int g0 = 0; g0 < nlist; g0 += 32) {
-                const int j = g0 + lane;
-                bool hit = false, near = false;
-                float4 st[3];
-                if (j < nlist) {
-                    const int r = regions ? (int)list[j] : j;
-                    hit = stage_pair(S.a[r], S.c[r], ox, oy, oz, hres, cull_ls2, st, &near);
-                }
-                // the staging of k_bgki: near rays first, two to a pair record, a pad ray last
-                const unsigned mnear = __ballot_sync(0xffffffffu, near);
-                const unsigned mfar = __ballot_sync(0xffffffffu, hit && !near);
-                const int nn = __popc(mnear), nh = nn + __popc(mfar);
-                if (hit) stage_put(stg, near ? __popc(mnear & lanes_below) : nn + __popc(mfar & lanes_below), st);
-                if ((nh & 1) && lane == 0) stage_pad(stg, nh);
-                __syncwarp();
-                const int npn = (nn + 1) >> 1, npa = (nh + 1) >> 1;
-                for (int k = 0; k < npn; ++k) {
-                    const float4* B = reinterpret_cast<const float4*>(stg + k * kStagePairFloats);
-                    {  // occupied term
-                        const float4 b4 = B[4], b5 = B[5];
-                        const F2 vx = add2(F2::of(b4.x, b4.y), DX), vy = add2(F2::of(b4.z, b4.w), DY);
-                        const F2 vz = add2(F2::of(b5.x, b5.y), DZ);
-                        const F2 d2o = fma2(vz, vz, fma2(vy, vy, mul2(vx, vx)));
-                        float oa, ob;
-                        d2o.split(oa, ob);
-                        const TabPos2 po = tab_pos2(d2o, TS);
-                        if (oa < ls2c) eval(po.a, fo, ho);
-                        if (ob < ls2c) eval(po.b, fo, ho);
-                    }
-                    F2 dp;
-                    const F2 d2f = free_d2x2(B[0], B[1], B[2], B[3], DX, DY, DZ, &dp);
-                    const float4 b5 = B[5];
-                    const F2 toend = add2(F2::of(b5.z, b5.w), dp);  // d_proj - d_m
-                    float fa, fb, ea, eb;
-                    d2f.split(fa, fb);
-                    toend.split(ea, eb);
-                    const TabPos2 pf = tab_pos2(d2f, TS);
-                    if (ea < 0.0f && fa < ls2c) eval(pf.a, ff, hf);
-                    if (eb < 0.0f && fb < ls2c) eval(pf.b, ff, hf);
-                }
-                for (int k = npn; k < npa; ++k) {
-                    const float4* B = reinterpret_cast<const float4*>(stg + k * kStagePairFloats);
-                    F2 dp;
-                    const F2 d2f = free_d2x2(B[0], B[1], B[2], B[3], DX, DY, DZ, &dp);
-                    float fa, fb;
-                    d2f.split(fa, fb);
-                    const TabPos2 pf = tab_pos2(d2f, TS);
-                    if (fa < ls2c) eval(pf.a, ff, hf);
-                    if (fb < ls2c) eval(pf.b, ff, hf);
-                }
-                __syncwarp();
-            }
-            if (L.c >= 0) {
-                unsigned long long* ac = acc4 + 4 * (long)(coff + L.c);
-                if (fo) atomicAdd(ac, (unsigned long long)fo);
-                if (ff) atomicAdd(ac + 1, (unsigned long long)ff);
-                if (ho) atomicAdd(ac + 2, (unsigned long long)ho);
-                if (hf) atomicAdd(ac + 3, (unsigned long long)hf);
-            }
-        }
-        __syncthreads();
-    }
+    CalibEval ev;
+    ev.ftab = tab;
+    ev.htab = tab + kKernelTabEntries;
+    ev.acc4 = acc4;
+    run_items(A, smem_raw + kCalibTabBytes, ev, [](const ItemConst&) {});
 }
 
 cudaError_t launch_bgki_sums(const Batch& bt, RayBuffers& rb, const float4* f_tab, const float4* dls_tab,
                              unsigned long long* acc4, DevStatus* status, int num_sms, cudaStream_t st) {
-    if (rb.chunk < 32 || rb.chunk > kChunk) return cudaErrorInvalidValue;
+    if (rb.chunk < 32 || rb.chunk > kCalibChunk) return cudaErrorInvalidValue;
     EvArgs A = make_args(bt, rb, CellState{}, CellWork{}, false, status);
     A.ktab = f_tab;
-    // 4 CTAs per SM with region lists up to kCalibChunk rays per item, else 3 without them
-    const bool small = rb.chunk <= kCalibChunk;
-    const size_t sm = calib_smem_bytes(rb.chunk, small);
-    auto kern = small ? k_bgki_sums<4, true> : k_bgki_sums<3>;
+    const size_t sm = calib_smem_bytes(rb.chunk);
     int per_sm = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kEvThreads, sm);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bgki_sums, kEvThreads, sm);
     ++g_launches;
-    kern<<<num_sms * std::max(1, per_sm), kEvThreads, sm, st>>>(A, dls_tab, acc4);
+    k_bgki_sums<<<num_sms * std::max(1, per_sm), kEvThreads, sm, st>>>(A, dls_tab, acc4);
     return cudaGetLastError();
 }
 
-// The K3DOM evidence launch is persistent: one CTA per resident slot of the build the chunk selects
-// (128 threads at <= 256 rays, 256 threads with region lists at <= 512, 256 threads at <= 1024).
+// The K3DOM evidence launch is persistent: one CTA per resident slot.
 struct BgkiLaunch {
-    int blocks, threads;
+    int blocks;
     size_t smem;
 };
 
@@ -1911,27 +2156,14 @@ static BgkiLaunch bgki_launch(int chunk) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     BgkiLaunch L;
-    if (chunk <= kSmallChunk) {
-        L.threads = kSmallWarps * 32;
-        L.smem = bgki_smem_bytes(chunk, kSmallWarps);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bgki<8, kSmallWarps * 32>, L.threads, L.smem);
-    } else if (chunk <= 512) {
-        L.threads = kEvThreads;
-        L.smem = bgki_smem_bytes(chunk, kEvWarps, true);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bgki<4, kEvThreads, true>, L.threads, L.smem);
-    } else {
-        L.threads = kEvThreads;
-        L.smem = bgki_smem_bytes(chunk);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bgki<3>, L.threads, L.smem);
-    }
+    L.smem = bgki_smem_bytes(chunk);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bgki, kEvThreads, L.smem);
     L.blocks = sms * std::max(1, per_sm);
     return L;
 }
 
 int k3dom_evidence_blocks(int chunk) { return bgki_launch(chunk).blocks; }
 
-// Work items of up to 512 rays leave shared memory for a fourth CTA per SM; that build is limited
-// to 64 registers. Items of up to 256 rays run in 128-thread CTAs, 8 per SM. Both builds compute the same sums (exactly), so the choice is speed only.
 cudaError_t launch_k3dom_evidence(const Batch& bt, RayBuffers& rb, CellState cs, CellWork cw, bool first_frame,
                                   DevStatus* status, cudaStream_t st, bool fuse_update) {
     if (rb.chunk < 32 || rb.chunk > kChunk) return cudaErrorInvalidValue;
@@ -1939,12 +2171,7 @@ cudaError_t launch_k3dom_evidence(const Batch& bt, RayBuffers& rb, CellState cs,
     A.fuse_update = fuse_update ? 1 : 0;
     const BgkiLaunch L = bgki_launch(rb.chunk);
     ++g_launches;
-    if (rb.chunk <= kSmallChunk)  // 128-thread CTAs: 8 per SM, each item's end waits on 4 warps
-        k_bgki<8, kSmallWarps * 32><<<L.blocks, L.threads, L.smem, st>>>(A);
-    else if (rb.chunk <= 512)
-        k_bgki<4, kEvThreads, true><<<L.blocks, L.threads, L.smem, st>>>(A);
-    else
-        k_bgki<3><<<L.blocks, L.threads, L.smem, st>>>(A);
+    k_bgki<<<L.blocks, kEvThreads, L.smem, st>>>(A);
     return cudaGetLastError();
 }
 
@@ -2146,20 +2373,11 @@ cudaError_t launch_ds_evidence(const Batch& bt, RayBuffers& rb, CellState cs, Ce
 long ds_count_bytes(long items) { return items * (long)kMaxTileCells; }
 
 cudaError_t evidence_init() {
-    cudaError_t e = cudaFuncSetAttribute(k_bgki<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_bgki, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)bgki_smem_bytes(kChunk));
     if (e != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_bgki<8, kSmallWarps * 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)bgki_smem_bytes(kSmallChunk, kSmallWarps))))
-        return e;
-    if ((e = cudaFuncSetAttribute(k_bgki<4, kEvThreads, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)bgki_smem_bytes(512, kEvWarps, true))))
-        return e;
-    if ((e = cudaFuncSetAttribute(k_bgki_sums<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)calib_smem_bytes(kChunk))))
-        return e;
-    if ((e = cudaFuncSetAttribute(k_bgki_sums<4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)calib_smem_bytes(kCalibChunk, true))))
+    if ((e = cudaFuncSetAttribute(k_bgki_sums, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)calib_smem_bytes(kCalibChunk))))
         return e;
     // 48 KB of copies plus the static barrier: above the default per-CTA limit
     return cudaFuncSetAttribute(k_k3dom_update_cells_bulk, cudaFuncAttributeMaxDynamicSharedMemorySize,
