@@ -521,6 +521,7 @@ cudaError_t alloc_ray_lane(k3dom_calib* c, RayBuffers& rb, int max_points, long 
     long cap = std::min(need + need / 4, 0xFFFFFFF0L);
     rb.capacity = cap;
     rb.chunk = kCalibChunk;
+    rb.item_slots = evidence_slots(c->num_sms);
     std::vector<void*>* L = &c->ray_allocs;
     cudaError_t e;
     if ((e = c->alloc(&rb.ray_a, N, L)) || (e = c->alloc(&rb.ray_c, N, L)) ||

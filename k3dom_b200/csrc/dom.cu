@@ -395,6 +395,7 @@ cudaError_t alloc_ray_buffers(k3dom_handle* h) {
     if (cap > 0xFFFFFFF0L) cap = 0xFFFFFFF0L;
     rb.capacity = cap;
     rb.chunk = h->chunk;
+    rb.item_slots = h->ds() ? 0 : evidence_slots(h->num_sms);
     const int N = h->N, T = h->T;
     if ((e = h->alloc(&rb.ray_a, N, true, L)) || (e = h->alloc(&rb.ray_c, N, true, L)) ||
         (e = h->alloc(&rb.counts, (size_t)kRayThreads * N, true, L)) || (e = h->alloc(&rb.evals2, cap, false, L)) ||

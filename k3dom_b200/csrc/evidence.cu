@@ -350,9 +350,27 @@ __global__ void k_tile_start(const uint32_t* __restrict__ skeys, const uint32_t*
     tile_start[t] = (uint32_t)lo;
 }
 
-__global__ void k_tile_items(const uint32_t* __restrict__ tile_start, int T, int chunk, uint32_t* __restrict__ items) {
+// Rays per work item of a frame with `entries` (tile, ray) entries: at most chunk, and so few that
+// every CTA slot of the evidence launch gets about kItemsPerSlot items (a multiple of 32 rays, kItemMin
+// at least: two full batches for a sub-block that all of them reach). slots = 0: always chunk. The
+// sums are exact, so the size changes no bit. With 1,024-ray items a small scan leaves most of the
+// GPU idle while a few CTAs walk long lists: 2,000 rays in 32x32x8 voxels, evidence 98 -> 27 us;
+// 30,000 rays in 64x64x16, 139 -> 106 us; 60,000 in 100x100x12, 158 -> 130 us. From about 1.2
+// million entries on nothing changes. Four or eight items per slot cost more staging than they
+// balance (30,000 rays: 111 and 128 us); 32 or 128 rays at least measured the same.
+constexpr int kItemsPerSlot = 2;
+constexpr int kItemMin = 64;
+__device__ __forceinline__ int item_rays(uint32_t entries, int chunk, int slots) {
+    if (slots <= 0) return chunk;
+    const uint32_t n = entries / (uint32_t)(slots * kItemsPerSlot);
+    return min(chunk, max(kItemMin, (int)((n + 31u) & ~31u)));
+}
+
+__global__ void k_tile_items(const uint32_t* __restrict__ tile_start, const uint32_t* __restrict__ total, int T,
+                             int max_chunk, int slots, uint32_t* __restrict__ items) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
+    const int chunk = item_rays(total[2], max_chunk, slots);
     const uint32_t len = tile_start[t + 1] - tile_start[t];
     items[t] = len == 0 ? 1u : (len + chunk - 1) / chunk;
 }
@@ -377,7 +395,8 @@ __global__ void k_finish_lists(const uint32_t* __restrict__ item_off, int T, Dev
 // tiles. On overflow (more entries than the list holds) every range is empty.
 constexpr int kRangeThreads = 1024;
 __global__ void __launch_bounds__(kRangeThreads)
-    k_tile_ranges(uint32_t* __restrict__ tile_tally, int T, int chunk, long capacity, uint32_t* __restrict__ tile_start,
+    k_tile_ranges(uint32_t* __restrict__ tile_tally, int T, int max_chunk, int slots, long capacity,
+                  uint32_t* __restrict__ tile_start,
                   uint32_t* __restrict__ item_off, uint32_t* __restrict__ total, DevStatus* status) {
     __shared__ unsigned long long sm[kRangeThreads / 32 + 1];
     const int per = (T + kRangeThreads - 1) / kRangeThreads;
@@ -387,6 +406,7 @@ __global__ void __launch_bounds__(kRangeThreads)
     unsigned long long entries;
     const unsigned long long base = block_exclusive_scan<unsigned long long, kRangeThreads>(n, sm, &entries);
     const bool over = entries > (unsigned long long)capacity;
+    const int chunk = item_rays(over ? 0u : (uint32_t)entries, max_chunk, slots);
     unsigned long long o = over ? 0ull : base;
     unsigned long long ni = 0;
     for (int t = t0; t < t1; ++t) {
@@ -551,7 +571,7 @@ cudaError_t build_ray_lists(const Batch& bt, const float* xs, const float* ys, c
         k_ray_count<true><<<blocks, kBlock, hist, st>>>(bt, xs, ys, zs, 0, rb.ray_a, rb.ray_c, rb.counts,
                                                          rb.tile_tally, rb.block_base, status);
         ++g_launches;
-        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.capacity, rb.tile_start,
+        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.capacity, rb.tile_start,
                                                    rb.item_off, rb.total, status);
         ++g_launches;
         k_ray_place<<<blocks, kBlock, hist, st>>>(bt, rb.ray_a, rb.counts, rb.tile_start, rb.block_base, rb.total,
@@ -579,7 +599,7 @@ cudaError_t build_ray_lists(const Batch& bt, const float* xs, const float* ys, c
     ++g_launches;
     k_tile_start<<<div_up(T + 1, kBlock), kBlock, 0, st>>>(rb.ekeys2, rb.total, T, rb.tile_start);
     ++g_launches;
-    k_tile_items<<<div_up(T, kBlock), kBlock, 0, st>>>(rb.tile_start, T, rb.chunk, rb.tile_items);
+    k_tile_items<<<div_up(T, kBlock), kBlock, 0, st>>>(rb.tile_start, rb.total, T, rb.chunk, rb.item_slots, rb.tile_items);
     e = scan_u32_exclusive(rb.tile_items, rb.item_off, T, rb.scan_tmp, rb.item_off + T, st);
     if (e != cudaSuccess) return e;
     ++g_launches;
@@ -707,6 +727,8 @@ struct EvArgs {
     const uint32_t* evals;
     const float4* ray_a;
     const double4* ray_c;
+    const uint32_t* total;  // [2]: entries in the lists
+    int item_slots;         // see item_rays
     const float4* ktab;  // S tables of kKernelTab entries, fixed-point scale folded in
     uint32_t* tile_done;
     unsigned long long* acc;
@@ -1590,8 +1612,9 @@ __device__ __forceinline__ void run_items(const EvArgs& A, unsigned char* smem, 
     const BgkiSmem S = bgki_smem(smem, A.chunk);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t total_items = A.item_off[A.bt.T];
+    const int chunk = item_rays(A.total[2], A.chunk, A.item_slots);
     for (;;) {
-        if (wid == 0) fetch_item(A, total_items, A.chunk, &I);
+        if (wid == 0) fetch_item(A, total_items, chunk, &I);
         if (threadIdx.x < kRegions) s_rcnt[threadIdx.x] = 0;
         if (threadIdx.x == kEvThreads - 1) s_next_sb = 0;
         __syncthreads();
@@ -2002,6 +2025,8 @@ static EvArgs make_args(const Batch& bt, RayBuffers& rb, CellState cs, CellWork 
     A.evals = rb.evals2;
     A.ray_a = rb.ray_a;
     A.ray_c = rb.ray_c;
+    A.total = rb.total;
+    A.item_slots = rb.item_slots;
     A.ktab = rb.ktab;
     A.tile_done = rb.tile_done;
     A.acc = rb.acc;
@@ -2161,6 +2186,8 @@ static BgkiLaunch bgki_launch(int chunk) {
     L.blocks = sms * std::max(1, per_sm);
     return L;
 }
+
+int evidence_slots(int num_sms) { return num_sms * kEvCtas; }
 
 int k3dom_evidence_blocks(int chunk) { return bgki_launch(chunk).blocks; }
 

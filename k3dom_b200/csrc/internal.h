@@ -155,7 +155,8 @@ struct RayBuffers {
     uint32_t* total;       // [0] = entries, [2] = entries kept (0 on overflow)
     long capacity;         // entries
     long ds_count_capacity;
-    int chunk;             // rays per work item
+    int chunk;             // largest number of rays per work item
+    int item_slots;        // CTA slots the work items are spread over (0: items of chunk rays whatever the scene)
 };
 long ray_entries_bound(const DevParams& p, const TileShape& ts, int max_points, float bin_R);
 // K3DOM ray lists are placed per tile through block histograms of all T tiles in shared memory
@@ -179,6 +180,8 @@ cudaError_t launch_k3dom_update_cells(const Batch& bt, RayBuffers& rb, CellState
                                       cudaStream_t st);
 cudaError_t launch_ds_evidence(const Batch& bt, RayBuffers& rb, CellState cs, CellWork cw, bool first_frame,
                                DevStatus* status, cudaStream_t st);
+// CTA slots of the K3DOM and calibration evidence kernels, for RayBuffers::item_slots.
+int evidence_slots(int num_sms);
 // CTAs of the K3DOM evidence launch for a chunk size (persistent grid).
 int k3dom_evidence_blocks(int chunk);
 // CTAs of the DS count pass and final pass (persistent: one per resident slot of each build).
