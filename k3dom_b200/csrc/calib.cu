@@ -445,6 +445,7 @@ struct k3dom_calib {
     int ray_points = 0;
     float ray_ls = 0.0f;  // length-scale the list capacity was sized for
     float4 *ftab = nullptr, *htab = nullptr;
+    cudaTextureObject_t ftex = 0;  // ftab through the texture path
     long long* acc = nullptr;        // F x C x 4 exact unit sums of the frames
     double* sums_out = nullptr;      // 4 x C staging of k3dom_calib_get_sums
     int sums_frames = 0;
@@ -467,6 +468,7 @@ struct k3dom_calib {
         return cudaMemsetAsync(*p, 0, std::max<size_t>(count, 1) * sizeof(T), st);
     }
     void release() {
+        if (ftex) cudaDestroyTextureObject(ftex);
         for (void* p : ray_allocs) cudaFree(p);
         for (void* p : allocs) cudaFree(p);
         ray_allocs.clear();
@@ -521,6 +523,7 @@ cudaError_t alloc_ray_lane(k3dom_calib* c, RayBuffers& rb, int max_points, long 
     long cap = std::min(need + need / 4, 0xFFFFFFF0L);
     rb.capacity = cap;
     rb.chunk = kCalibChunk;
+    rb.ktex = c->ftex;
     rb.item_slots = evidence_slots(c->num_sms);
     std::vector<void*>* L = &c->ray_allocs;
     cudaError_t e;
@@ -626,8 +629,8 @@ k3dom_status compute_sums(k3dom_calib* c, float ls) {
             if ((e = build_ray_lists(bt, f.pts, f.pts + f.n, f.pts + 2 * (long)f.n, c->rb[l], false, c->status + l,
                                      SortWait(), sk)))
                 return c->fail(e);
-            if ((e = launch_bgki_sums(bt, c->rb[l], c->ftab, c->htab, reinterpret_cast<unsigned long long*>(acc_k),
-                                      c->status + l, c->num_sms, sk)))
+            if ((e = launch_bgki_sums(bt, c->rb[l], c->htab, reinterpret_cast<unsigned long long*>(acc_k), c->status + l,
+                                      c->num_sms, sk)))
                 return c->fail(e);
         }
     }
@@ -749,6 +752,10 @@ k3dom_status k3dom_calib_create(const k3dom_params* base, int device, k3dom_cali
         (e = c->alloc(&c->htab, kKernelTableSize)) || (e = c->alloc(&c->sums_out, 4 * (size_t)d.C)) ||
         (e = c->alloc(&c->red, 6)))
         return bail(e);
+    RayBuffers tex{};
+    tex.ktab = c->ftab;
+    if ((e = make_kernel_table_texture(tex, 1))) return bail(e);
+    c->ftex = tex.ktex;
     std::vector<float4> ft(kKernelTableSize), ht(kKernelTableSize);
     build_calib_tables(ft.data(), ht.data());
     if ((e = cudaMemcpyAsync(c->ftab, ft.data(), sizeof(float4) * ft.size(), cudaMemcpyHostToDevice, c->st)) ||

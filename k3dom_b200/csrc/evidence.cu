@@ -729,7 +729,6 @@ struct EvArgs {
     const double4* ray_c;
     const uint32_t* total;  // [2]: entries in the lists
     int item_slots;         // see item_rays
-    const float4* ktab;  // S tables of kKernelTab entries, fixed-point scale folded in
     uint32_t* tile_done;
     unsigned long long* acc;
     uint8_t* ds_counts;
@@ -740,7 +739,7 @@ struct EvArgs {
     int first_frame;
     int chunk;  // rays per work item (<= kChunk)
     int fuse_update;  // K3DOM: the last CTA of a tile updates its cells (else k_k3dom_update_cells)
-    cudaTextureObject_t ktex;  // ktab through the texture path
+    cudaTextureObject_t ktex;  // the scenes' kernel tables (K3DOM), f's table (calibration)
 };
 
 // ================================================================ K3DOM
@@ -2027,7 +2026,6 @@ static EvArgs make_args(const Batch& bt, RayBuffers& rb, CellState cs, CellWork 
     A.ray_c = rb.ray_c;
     A.total = rb.total;
     A.item_slots = rb.item_slots;
-    A.ktab = rb.ktab;
     A.tile_done = rb.tile_done;
     A.acc = rb.acc;
     A.ds_counts = rb.ds_counts;
@@ -2081,13 +2079,16 @@ void build_calib_tables(float4* f_tab, float4* dls_tab) {
     build_table(unit_kernel_dls, 1.0, dls_tab);
 }
 
-// The calibration's values: f and -x f' from two tables in shared memory (through the texture path
-// they measured slower), two sums per evidence kind. f is clamped at 0 by FMA.SAT, -x f' lies in
-// [-3e-7, 0.78].
+// The calibration's values: f from its table through the texture path, -x f' from one in shared
+// memory, two sums per evidence kind. f is clamped at 0 by FMA.SAT, -x f' lies in [-3e-7, 0.78].
+// The kernel is bound by these gathers, and the two paths run side by side: gradient step at
+// 256x256x32 voxels with two 120,000-ray frames, 3.75 ms with both tables in shared memory, 3.96 ms
+// with both through the texture path, 3.50 ms with one in each.
 static_assert(kCalibShift == kFxShift, "units of the calibration sums");
 
 struct CalibEval {
-    const float4 *ftab, *htab;  // [kKernelTabEntries] each
+    cudaTextureObject_t tex;  // f
+    const float4* htab;       // [kKernelTabEntries] -x f'
     unsigned long long* acc4;
     FxSum fo[4], ff[4], ho[4], hf[4], occ_f, occ_h;
     int n_occ, n_free;
@@ -2110,7 +2111,7 @@ struct CalibEval {
         n_occ += steps;
     }
     __device__ __forceinline__ void value(const TabPos& q, float* f, float* h) {
-        const float4 c = ftab[q.i], d = htab[q.i];
+        const float4 c = tex1Dfetch<float4>(tex, q.i), d = htab[q.i];
         *f = __saturatef(fmaf(q.f, fmaf(q.f, fmaf(q.f, c.w, c.z), c.y), c.x));
         *h = fmaf(q.f, fmaf(q.f, fmaf(q.f, d.w, d.z), d.y), d.x);
     }
@@ -2135,7 +2136,7 @@ struct CalibEval {
     }
 };
 
-constexpr size_t kCalibTabBytes = (2 * sizeof(float4) * kKernelTabEntries + 31) & ~(size_t)31;
+constexpr size_t kCalibTabBytes = (sizeof(float4) * kKernelTabEntries + 31) & ~(size_t)31;
 
 inline size_t calib_smem_bytes(int chunk) { return kCalibTabBytes + bgki_smem_bytes(chunk); }
 
@@ -2145,23 +2146,19 @@ inline size_t calib_smem_bytes(int chunk) { return kCalibTabBytes + bgki_smem_by
 __global__ void __launch_bounds__(kEvThreads, kEvCtas) k_bgki_sums(EvArgs A, const float4* __restrict__ htab,
                                                                unsigned long long* __restrict__ acc4) {
     extern __shared__ __align__(32) unsigned char smem_raw[];
-    float4* tab = reinterpret_cast<float4*>(smem_raw);
-    for (int i = threadIdx.x; i < kKernelTabEntries; i += kEvThreads) {  // used after run_items' first barrier
-        tab[i] = A.ktab[i];
-        tab[kKernelTabEntries + i] = htab[i];
-    }
+    float4* tab = reinterpret_cast<float4*>(smem_raw);  // used after run_items' first barrier
+    for (int i = threadIdx.x; i < kKernelTabEntries; i += kEvThreads) tab[i] = htab[i];
     CalibEval ev;
-    ev.ftab = tab;
-    ev.htab = tab + kKernelTabEntries;
+    ev.tex = A.ktex;
+    ev.htab = tab;
     ev.acc4 = acc4;
     run_items(A, smem_raw + kCalibTabBytes, ev, [](const ItemConst&) {});
 }
 
-cudaError_t launch_bgki_sums(const Batch& bt, RayBuffers& rb, const float4* f_tab, const float4* dls_tab,
-                             unsigned long long* acc4, DevStatus* status, int num_sms, cudaStream_t st) {
+cudaError_t launch_bgki_sums(const Batch& bt, RayBuffers& rb, const float4* dls_tab, unsigned long long* acc4,
+                             DevStatus* status, int num_sms, cudaStream_t st) {
     if (rb.chunk < 32 || rb.chunk > kCalibChunk) return cudaErrorInvalidValue;
     EvArgs A = make_args(bt, rb, CellState{}, CellWork{}, false, status);
-    A.ktab = f_tab;
     const size_t sm = calib_smem_bytes(rb.chunk);
     int per_sm = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_bgki_sums, kEvThreads, sm);

@@ -130,7 +130,7 @@ struct RayBuffers {
     float4* ray_a;         // m.x, m.y, m.z, d_m (K3DOM) | |m|^2 (DS)
     double4* ray_c;        // d_m, margin, 1/d_m, 0 in FP64 (K3DOM)
     float4* ktab;          // per scene: sparse-kernel table with the fixed-point scale folded in
-    cudaTextureObject_t ktex;  // ktab read through the texture path (k_bgki), 0 when not made
+    cudaTextureObject_t ktex;  // the kernel table through the texture path (k_bgki: ktab; k_bgki_sums: f), 0 when not made
     uint32_t* counts;      // [kRayThreads * N] tiles touched per point slot (DS) or per thread of a slot
     uint32_t* offsets;     // exclusive scan of counts (DS)
     uint32_t* ekeys;       // entries: global tile id (DS)
@@ -192,13 +192,14 @@ cudaError_t evidence_init();
 // zero entry at u = 1 (513 float4), so an index taken at the support's edge needs no clamp.
 void build_kernel_table(float sigma, double scale, float4* out);
 constexpr int kKernelTableSize = 513;
-// Rays per calibration work item: the largest chunk whose evidence-sums build keeps 4 CTAs per
-// SM with its per-region ray lists in shared memory.
-constexpr int kCalibChunk = 448;
+// Rays per calibration work item at most: 4 CTAs per SM still fit beside the derivative's table
+// (gradient step at 256x256x32 voxels: 448 rays 3.90 ms, 768 rays 3.75 ms).
+constexpr int kCalibChunk = 768;
 // Calibration: unit-amplitude kernel and -x f'(x) tables scaled to units of 2^-kCalibShift.
 constexpr int kCalibShift = 40;
 void build_calib_tables(float4* f_tab, float4* dls_tab);
-cudaError_t launch_bgki_sums(const Batch& bt, RayBuffers& rb, const float4* f_tab, const float4* dls_tab,
-                             unsigned long long* acc4, DevStatus* status, int num_sms, cudaStream_t st);
+// rb.ktex: f's table; dls_tab: the table of -x f'.
+cudaError_t launch_bgki_sums(const Batch& bt, RayBuffers& rb, const float4* dls_tab, unsigned long long* acc4,
+                             DevStatus* status, int num_sms, cudaStream_t st);
 
 }  // namespace k3dom
