@@ -427,8 +427,11 @@ cudaError_t alloc_ray_buffers(k3dom_handle* h) {
     if (h->ds()) {
         h->ds_sized_chunk = std::max(32, h->chunk);
         const long items_max = T + cap / h->ds_sized_chunk + 2;
-        rb.ds_count_capacity = ds_count_bytes(items_max);
-        if ((e = h->alloc(&rb.ds_counts, rb.ds_count_capacity, true, L))) return e;
+        rb.ds_stride = 1;
+        for (const SceneHost& x : h->sc) rb.ds_stride = std::max(rb.ds_stride, x.ts.tx * x.ts.ty * x.ts.tz);
+        rb.ds_capacity = items_max * rb.ds_stride;
+        if ((e = h->alloc(&rb.ds_counts, rb.ds_capacity, false, L)) || (e = h->alloc(&rb.ds_r2, rb.ds_capacity, false, L)))
+            return e;
     }
     rb.os_words = onesweep_scratch_words(cap, bits);
     rb.scan_words = scan_u32_tiles(std::max((long)N, (long)T + 1)) + 16;
@@ -710,8 +713,10 @@ cudaError_t enq_binning(k3dom_handle* h, cudaStream_t s) {
 
 cudaError_t enq_evidence(k3dom_handle* h, bool first_frame) {
     const Batch bt = h->batch();
-    if (h->ds())
-        return launch_ds_evidence(bt, h->rb, h->cells(), h->cw, first_frame, h->status, h->st);
+    if (h->ds()) {
+        const cudaError_t e = launch_ds_measure(bt, h->rb, h->status, h->st);
+        return e ? e : launch_ds_update(bt, h->rb, h->cells(), h->cw, first_frame, h->status, h->st);
+    }
     return launch_k3dom_evidence(bt, h->rb, h->cells(), h->cw, first_frame, h->status, h->st);
 }
 
@@ -803,17 +808,15 @@ cudaError_t enq_frame(k3dom_handle* h) {
     if ((e = enq_draws(h, h->st2))) return e;
     if ((e = cudaEventRecord(h->ev_join, h->st2))) return e;
     // the ray lists depend on the points only: built beside prediction and assignment, except
-    // when each stage is timed on its own. K3DOM's evidence needs only the lists, so it runs there
-    // too, and the cells are updated once both sides are done; DS's evidence pass needs the
-    // particles' per-cell counts throughout and follows assignment.
+    // when each stage is timed on its own. The evidence (K3DOM) and the measurement grid (DS) need
+    // only the lists, so they run there too, and the cells are updated once both sides are done.
     const bool overlap = !h->timing;
-    const bool split = overlap && !h->ds();
     if (overlap) {
         if ((e = cudaStreamWaitEvent(h->st3, h->ev_fork, 0))) return e;
         if ((e = enq_binning(h, h->st3))) return e;
-        if (split && (e = launch_k3dom_evidence(h->batch(), h->rb, h->cells(), h->cw, false, h->status, h->st3,
-                                                false)))
-            return e;
+        e = h->ds() ? launch_ds_measure(h->batch(), h->rb, h->status, h->st3)
+                    : launch_k3dom_evidence(h->batch(), h->rb, h->cells(), h->cw, false, h->status, h->st3, false);
+        if (e) return e;
         if ((e = cudaEventRecord(h->ev_bin, h->st3))) return e;
     }
     rec(h, 0);
@@ -821,12 +824,11 @@ cudaError_t enq_frame(k3dom_handle* h) {
     rec(h, 1);
     if ((e = enq_assign(h))) return e;
     rec(h, 2);
-    if (split) {
+    if (overlap) {
         if ((e = cudaStreamWaitEvent(h->st, h->ev_bin, 0))) return e;
-        if ((e = launch_k3dom_update_cells(h->batch(), h->rb, h->cells(), h->cw, h->status, h->st))) return e;
-    } else if (overlap) {
-        if ((e = cudaStreamWaitEvent(h->st, h->ev_bin, 0))) return e;
-        if ((e = enq_evidence(h, false))) return e;
+        e = h->ds() ? launch_ds_update(h->batch(), h->rb, h->cells(), h->cw, false, h->status, h->st)
+                    : launch_k3dom_update_cells(h->batch(), h->rb, h->cells(), h->cw, h->status, h->st);
+        if (e) return e;
     } else if ((e = enq_occupancy(h, false))) {
         return e;
     }
@@ -1391,7 +1393,7 @@ k3dom_status k3dom_get_tuning(k3dom_handle* h, k3dom_tuning* out) {
     for (int k = 0; k < kTuneCount && k < (int)h->tune_ms.size() && k < K3DOM_TUNE_MAX_CANDIDATES; ++k)
         out->candidate_ms[k] = h->tune_ms[k];
     if (h->ds()) {
-        k3dom_ds_evidence_blocks(&out->evidence_count_blocks, &out->evidence_blocks);
+        k3dom_ds_evidence_blocks(&out->evidence_blocks, &out->evidence_count_blocks);
     } else {
         out->evidence_blocks = k3dom_evidence_blocks(h->rb.chunk);
         out->evidence_count_blocks = 0;

@@ -19,8 +19,8 @@
 // its first-100 rule needs. One CTA takes one (tile, chunk of rays) work item
 // from a device work counter and stages the chunk's rays in shared memory; its warps pull the
 // tile's 4x4x2-cell sub-blocks from a block-local counter and cull 32 rays at a time with one
-// ballot. K3DOM collects the surviving rays into batches of 32, resolves them in FP64 and evaluates
-// two rays at a time for four cells per lane; DS evaluates each ray for every lane's own cell.
+// ballot, collect the surviving rays into batches of 32, resolve them in FP64 and evaluate two rays
+// at a time for four cells per lane. DS walks each ray's cells (see k_ds_rays).
 //
 // K3DOM evidence is summed in fixed point: each kernel value is rounded once to an integer
 // number of units of 2^-k sigma (the table carries the scale), summed exactly in 64-bit
@@ -48,7 +48,7 @@ static_assert(kKernelTabEntries == kKernelTableSize, "kernel table size");
 constexpr int kEvThreads = 256;
 constexpr int kEvWarps = kEvThreads / 32;
 constexpr int kEvCtas = 4;  // K3DOM evidence CTAs per SM: 64 registers a thread
-constexpr int kDsMaxNeighbors = 100;  // measurement_grid.cu:87
+constexpr uint32_t kDsMaxNeighbors = 100;  // measurement_grid.cu:87
 constexpr int kFxShift = 40;  // fixed-point units of the K3DOM and calibration sums: 2^-40 of the scaled kernel
 
 // ================================================================ binning
@@ -608,23 +608,6 @@ cudaError_t build_ray_lists(const Batch& bt, const float* xs, const float* ys, c
 }
 
 // ================================================================ shared kernel machinery
-__device__ __forceinline__ int find_tile(const uint32_t* __restrict__ item_off, int T, uint32_t item) {
-    // last t with item_off[t] <= item
-    int lo = 0, hi = T;  // answer in [0, T)
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (item_off[mid] <= item) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
-struct CellLoc {
-    int c;          // cell index within the scene, -1 when outside the grid
-    int local;      // cell index within the tile
-    float x, y, z;  // cell centre relative to the sensor [m], reference FP32 operation order
-    float ox, oy, oz;  // anchor: centre of the sub-block's cell (2, 2, 1), same formula
-};
-
 // Cell centre of index triple (ix, iy, iz), the expression of mass_update.cu:92-99 /
 // measurement_grid.cu:77-84 evaluated in FP32 in the reference's order.
 __device__ __forceinline__ void centre_xyz(int ix, int iy, int iz, const DevParams& p, float sx, float sy, float sz,
@@ -643,22 +626,6 @@ __device__ __forceinline__ SbCell sb_cell(const TileShape& ts, int t, int sb) {
     const int tx = t % ts.ntx, ty = (t / ts.ntx) % ts.nty, tz = t / (ts.ntx * ts.nty);
     const int sbx = sb % ts.nsbx, sby = (sb / ts.nsbx) % ts.nsby, sbz = sb / (ts.nsbx * ts.nsby);
     return SbCell{tx * ts.tx + sbx * 4, ty * ts.ty + sby * 4, tz * ts.tz + sbz * 2};
-}
-
-__device__ __forceinline__ CellLoc locate(const DevParams& p, const TileShape& ts, int t, int sb, int lane,
-                                          float sx, float sy, float sz) {
-    const int tx = t % ts.ntx, ty = (t / ts.ntx) % ts.nty, tz = t / (ts.ntx * ts.nty);
-    const int sbx = sb % ts.nsbx, sby = (sb / ts.nsbx) % ts.nsby, sbz = sb / (ts.nsbx * ts.nsby);
-    const int lx = sbx * 4 + (lane & 3), ly = sby * 4 + ((lane >> 2) & 3), lz = sbz * 2 + (lane >> 4);
-    const int ix = tx * ts.tx + lx, iy = ty * ts.ty + ly, iz = tz * ts.tz + lz;
-    CellLoc L;
-    L.local = lx + ts.tx * (ly + ts.ty * lz);
-    const bool in = ix < p.G && iy < p.G && iz < p.Gz;
-    L.c = in ? ix + p.G * iy + p.G * p.G * iz : -1;
-    centre_xyz(ix, iy, iz, p, sx, sy, sz, &L.x, &L.y, &L.z);
-    centre_xyz(tx * ts.tx + sbx * 4 + 2, ty * ts.ty + sby * 4 + 2, tz * ts.tz + sbz * 2 + 1, p, sx, sy, sz, &L.ox,
-               &L.oy, &L.oz);
-    return L;
 }
 
 // Sub-blocks go to the warps nearest to the sensor first. A sub-block's work grows with the rays
@@ -699,27 +666,6 @@ __device__ __forceinline__ void sb_order_rank(SbOrder& o, int nsb) {
 
 __device__ __forceinline__ int sb_at(const SbOrder& o, int n, int nsb) { return nsb > kMaxOrderedSb ? n : o.idx[n]; }
 
-// The work item a CTA holds: its tile (global and scene-local), scene and ray range.
-struct Item {
-    int t, lt, sc;
-    uint32_t k, n_items, e0;
-    int nr;
-};
-
-__device__ __forceinline__ Item item_of(const Batch& bt, const uint32_t* item_off, const uint32_t* tile_start,
-                                        uint32_t item, int chunk) {
-    Item it;
-    it.t = find_tile(item_off, bt.T, item);
-    it.sc = scene_of(bt.off->tile, bt.S, it.t);
-    it.lt = it.t - bt.off->tile[it.sc];
-    it.k = item - item_off[it.t];
-    it.n_items = item_off[it.t + 1] - item_off[it.t];
-    it.e0 = tile_start[it.t] + it.k * (uint32_t)chunk;
-    const uint32_t e1 = min(tile_start[it.t + 1], it.e0 + (uint32_t)chunk);
-    it.nr = (int)(e1 > it.e0 ? e1 - it.e0 : 0);
-    return it;
-}
-
 struct EvArgs {
     Batch bt;
     const uint32_t* item_off;
@@ -731,8 +677,10 @@ struct EvArgs {
     int item_slots;         // see item_rays
     uint32_t* tile_done;
     unsigned long long* acc;
+    uint32_t* ds_r2;
     uint8_t* ds_counts;
-    long ds_count_capacity;
+    long ds_capacity;
+    int ds_stride;
     CellState cs;
     CellWork cw;
     DevStatus* status;
@@ -983,12 +931,30 @@ __device__ __forceinline__ unsigned region_mask(float ax, float ay, float az, fl
 struct ItemConst {
     int live;  // 0: no item left
     int t, lt, nr, nsb, regions, coff, tbase;
-    uint32_t e0, n_items;
+    uint32_t item, e0, n_items;
     TileShape ts;
     int sc, G, Gz;
     float res, sx, sy, sz;
     float bin_R, ls2, tscale, rls2, rls;
 };
+
+// The tile of a work item: last t in [0, T) with item_off[t] <= item, 32 probes a step (the calling
+// warp, item the same in every lane).
+__device__ __forceinline__ int warp_find_tile(const uint32_t* __restrict__ item_off, int T, uint32_t item) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = T;
+    while (hi - lo > 1) {
+        const int span = hi - lo;
+        const int pos = span <= 33 ? min(lo + 1 + lane, hi) : lo + (int)((long)(lane + 1) * span / 33);
+        const unsigned m = __ballot_sync(0xffffffffu, pos < hi && item_off[pos] <= item);
+        const int n = __popc(m);  // a prefix of the lanes
+        const int at = __shfl_sync(0xffffffffu, pos, n > 0 ? n - 1 : 0);
+        const int up = __shfl_sync(0xffffffffu, pos, n < 32 ? n : 31);
+        if (n > 0) lo = at;
+        if (n < 32) hi = min(hi, up);
+    }
+    return lo;
+}
 
 // Takes the next work item (the calling warp only).
 __device__ __forceinline__ void fetch_item(const EvArgs& A, uint32_t total_items, int chunk, ItemConst* I) {
@@ -1001,20 +967,10 @@ __device__ __forceinline__ void fetch_item(const EvArgs& A, uint32_t total_items
         if (lane == 0) I->live = 0;
         return;
     }
-    // the tile: last t with item_off[t] <= item, 32 probes a step
-    int lo = 0, hi = bt.T;
-    while (hi - lo > 1) {
-        const int span = hi - lo;
-        const int pos = span <= 33 ? min(lo + 1 + lane, hi) : lo + (int)((long)(lane + 1) * span / 33);
-        const unsigned m = __ballot_sync(0xffffffffu, pos < hi && A.item_off[pos] <= item);
-        const int n = __popc(m);  // a prefix of the lanes
-        const int at = __shfl_sync(0xffffffffu, pos, n > 0 ? n - 1 : 0);
-        const int up = __shfl_sync(0xffffffffu, pos, n < 32 ? n : 31);
-        if (n > 0) lo = at;
-        if (n < 32) hi = min(hi, up);
-    }
+    const int lo = warp_find_tile(A.item_off, bt.T, item);
     if (lane != 0) return;
     I->live = 1;
+    I->item = item;
     I->t = lo;
     I->sc = scene_of(bt.off->tile, bt.S, lo);
     I->lt = lo - bt.off->tile[I->sc];
@@ -1792,225 +1748,403 @@ __device__ __forceinline__ bool ds_is_neighbor(float x, float y, float z, float 
     return ip > 0.0f && __fsub_rn(acs, __fdiv_rn(__fmul_rn(ip, ip), m.w)) < wr2;
 }
 
-// pOcc (measurement_grid.cu:28-39)
-__device__ __forceinline__ float ds_pocc(float x, float y, float z, float4 m, float delta) {
+// pOcc (measurement_grid.cu:28-39) from the squared distance between cell centre and point.
+__device__ __forceinline__ float ds_r_sqr(float x, float y, float z, float4 m) {
     const float dx = __fsub_rn(x, m.x), dy = __fsub_rn(y, m.y), dz = __fsub_rn(z, m.z);
-    const float r_sqr = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+    return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+}
+__device__ __forceinline__ float ds_pocc(float r_sqr, float delta) {
     const float delta_sqr = __fmul_rn(delta, delta);
     return __fmul_rn(0.95f, expf(__fdiv_rn(__fmul_rn(-0.5f, r_sqr), delta_sqr)));
 }
 
-// Pass COUNT (multi-chunk tiles, every chunk but the last): per (item, cell) number of
-// neighbours. Pass !COUNT: each cell takes its first (100 - neighbours in earlier chunks)
-// neighbours of the chunk, in list order, so the kept set is the reference's first 100 rays in
-// input order (measurement_grid.cu:86-97). Per-chunk summaries (any neighbour, all farther,
-// largest pOcc) are combined per cell with integer atomics; the last CTA of a tile runs the
-// measurement-to-mass step for the whole tile.
+// The measurement grid by rays. A ray's half-line meets about 300 cells of a 256x256x32 grid, 4 of
+// the 32 in a sub-block that it passes, so one lane per cell leaves most lanes idle; here one lane
+// takes one ray of a work item and walks the cells around the half-line inside the item's tile,
+// applies the reference's FP32 neighbour test to each and adds an accepted one to the cell's summary
+// in shared memory with two atomics. The summary is order-free: pOcc falls with the distance (every
+// operation of ds_pocc is monotone; expf was checked over all floats of [-110, 0]), so its maximum
+// over the neighbours is pOcc of the smallest squared distance, kept as float bits (>= 0) by an
+// integer minimum; beside it the number of neighbours and of those closer to the sensor than the
+// cell. Only the reference's first-100 rule (measurement_grid.cu:86-97) depends on the input order,
+// and only for cells with more than 100 neighbours. A tile's items hold its rays in input order, so
+// the items before the hundredth neighbour count in full, and the one that holds it is walked again
+// in order, by a warp, for that cell alone (k_ds_partial).
+//   k_ds_rays     per item: summaries; a tile with one item writes its cells' totals, the others
+//                 write per (item, cell) summaries; cells past 100 go to the worklist
+//   k_ds_combine  cells of tiles with several items: the items in order up to the hundredth neighbour
+//   k_ds_partial  the worklist
+//   k_ds_update   the measurement-to-mass step and the Dempster update of every cell
+// 256x256x32 voxels at 0.1 m, 120,000 rays: the lane-per-cell passes took 0.65 + 1.10 ms, these 0.62 +
+// 0.07 + 0.04 + 0.05 ms; 200x200x25 at 0.2 m, 60,000 rays: 0.69 -> 0.33 ms. k_ds_rays is bound by
+// instruction issue and by its waits at the items' ends (1,560 thread instructions per (tile, ray)
+// entry; 20 of 32 lanes in the layers' loops). One ray per lane with the layers as a loop ran at 6 of
+// 32 lanes (1.52 ms), one (ray, layer) per lane with plain loops over its cells 0.86 ms; CTAs of 128
+// or 64 threads wait less but leave longer tails (0.87 and 1.10 ms).
 constexpr int kMaxTileCells = 16 * 16 * 8;
+constexpr uint32_t kDsNone = 0xFFFFFFFFu;
+constexpr uint32_t kDsCloser = 0x10000u;  // in a cell's counter: neighbours | closer ones << 16
+static_assert(kChunk < 0x10000, "an item's count fits 16 bits");
 
-template <bool COUNT>
-__global__ void __launch_bounds__(kEvThreads, COUNT ? 5 : 4) k_dsgrid(EvArgs A) {
-    __shared__ float4 sa[kChunk];  // (m, |m|^2)
-    __shared__ float4 su[kChunk];  // (m / |m|, 0)
-    __shared__ uint16_t s_cand[kEvWarps][32];
-    __shared__ uint16_t s_reg[kRegions][kChunk];  // region lists, in input order
-    __shared__ int s_wq[2][kEvWarps][kRegions];     // per-warp region counts of a staging step
-    __shared__ int s_rcnt[kRegions];
-    __shared__ uint32_t s_item;
-    __shared__ int s_next_sb, s_last;
-    __shared__ SbOrder s_order;
+// Per-cell results in the evidence accumulators' memory (4 words per cell).
+struct DsCells {
+    uint32_t *r2, *flags, *work_cell, *work_item;  // flags: 1 any neighbour, 2 one closer than the cell
+    __device__ __forceinline__ DsCells(const EvArgs& A) {
+        r2 = reinterpret_cast<uint32_t*>(A.acc);
+        flags = r2 + A.bt.C;
+        work_cell = flags + A.bt.C;
+        work_item = work_cell + A.bt.C;
+    }
+};
+
+struct DsTile {
+    float2 c[3][16];  // cell-centre coordinate and its square, per axis
+    int o[3], n[3];   // first cell and number of cells inside the grid
+    uint32_t cf[kMaxTileCells], r2[kMaxTileCells];
+};
+
+// A ray's line through a tile, in layers along its axis A (x or y, whichever is larger; z for rays
+// steeper than that): at layer i (cells from the tile's first one) it crosses the layer at
+// B = pb + sb i, C = pc + sc i, and the cells of the layer within the window of the line form an
+// ellipse with half-extents eb = R sqrt(1 + sb^2) and ec along B and C. (B, C) is (y, z), (x, z) or
+// (x, y), so that the reference's sums over x, y, z are (A + B) + C, or (B + C) + A for axis z.
+struct DsRay {
+    float4 line;  // pb, sb, pc, sc
+    float4 ext;   // eb, ec, 1 / |m|^2, axis
+    float4 m;     // m, |m|^2
+};
+struct DsWarp {
+    DsRay ray[32];
+    uint16_t layer[32 * 16];  // lane of the ray | layer << 5
+};
+
+// Lays out the line of ray m and returns its range of layers (none: hi < lo). Distances are formed in
+// cell-index space; R carries the slack of the reference's FP32 test and of this arithmetic. A
+// neighbour needs a positive projection, which lies within 1.3 cells of its layer's crossing.
+__device__ __forceinline__ int2 ds_line(const DsTile& S, const float a[3], float4 m, float R, DsRay* out) {
+    const float il = rsqrtf(m.w);
+    const float ux = m.x * il, uy = m.y * il, uz = m.z * il;
+    const float hx = fabsf(ux), hy = fabsf(uy);
+    const int ax = fabsf(uz) > fmaxf(hx, hy) ? 2 : (hx >= hy ? 0 : 1);
+    const float uA = ax == 0 ? ux : (ax == 1 ? uy : uz), uB = ax == 0 ? uy : ux, uC = ax == 2 ? uy : uz;
+    const int B = ax == 0 ? 1 : 0, C = ax == 2 ? 1 : 2;
+    const float aA = sel3(a[0], a[1], a[2], ax), aB = sel3(a[0], a[1], a[2], B), aC = sel3(a[0], a[1], a[2], C);
+    const float iu = 1.0f / uA, sb = uB * iu, sc = uC * iu;
+    const float eb = R * sqrtf(fmaf(sb, sb, 1.0f)), ec = R * sqrtf(fmaf(sc, sc, 1.0f));
+    const float a0 = (float)S.o[ax] - aA;
+    const float pb = aB - (float)S.o[B] + sb * a0, pc = aC - (float)S.o[C] + sc * a0;
+    float lo = 0.0f, hi = (float)(S.n[ax] - 1);
+    if (uA > 0.0f) lo = fmaxf(lo, -a0 - 2.0f); else hi = fminf(hi, -a0 + 2.0f);
+    // layers where the line is inside the tile's B and C ranges
+    if (fabsf(sb) > 1e-3f) {
+        const float is = 1.0f / sb, t0 = (-eb - pb) * is, t1 = ((float)(S.n[B] - 1) + eb - pb) * is;
+        lo = fmaxf(lo, fminf(t0, t1) - 0.05f);
+        hi = fminf(hi, fmaxf(t0, t1) + 0.05f);
+    }
+    if (fabsf(sc) > 1e-3f) {
+        const float is = 1.0f / sc, t0 = (-ec - pc) * is, t1 = ((float)(S.n[C] - 1) + ec - pc) * is;
+        lo = fmaxf(lo, fminf(t0, t1) - 0.05f);
+        hi = fminf(hi, fmaxf(t0, t1) + 0.05f);
+    }
+    out->line = make_float4(pb, sb, pc, sc);
+    out->ext = make_float4(eb, ec, 1.0f / m.w, __int_as_float(ax));
+    out->m = m;
+    return make_int2((int)ceilf(lo), (int)floorf(hi));
+}
+
+// The candidate cells of one layer of one ray. STEEP: axis z.
+template <bool STEEP>
+__device__ __forceinline__ void ds_layer(DsTile& S, const TileShape& ts, const DsRay& r, int ax, int i, float wr2) {
+    const float4 ln = r.line, ex = r.ext, m = r.m;
+    const int B = STEEP ? 0 : 1 - ax, C = STEEP ? 1 : 2;
+    const float qb = fmaf(ln.y, (float)i, ln.x), qc = fmaf(ln.w, (float)i, ln.z);
+    const int b0 = max((int)ceilf(qb - ex.x), 0), b1 = min((int)floorf(qb + ex.x), S.n[B] - 1);
+    const int c0 = max((int)ceilf(qc - ex.y), 0), c1 = min((int)floorf(qc + ex.y), S.n[C] - 1);
+    const int stA = STEEP ? ts.tx * ts.ty : (ax == 0 ? 1 : ts.tx), stB = STEEP ? 1 : (ax == 0 ? ts.tx : 1);
+    const int stC = STEEP ? ts.tx : ts.tx * ts.ty;
+    const float mA = STEEP ? m.z : (ax == 0 ? m.x : m.y), mB = STEEP ? m.x : (ax == 0 ? m.y : m.x);
+    const float mC = STEEP ? m.y : m.z;
+    const float2 va = S.c[STEEP ? 2 : ax][i];
+    const float pa = __fmul_rn(va.x, mA), da = __fsub_rn(va.x, mA), dda = __fmul_rn(da, da);
+    // the layer's cells in blocks of 3 x 2 (nearly always one: the window is 1.73 cells wide across the
+    // ray and C slopes little for LiDAR rays), unrolled so that the six tests overlap
+    for (int cb = c0; cb <= c1; cb += 2) {
+        float2 vc[2];
+        float pc[2], ddc[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            vc[k] = S.c[C][min(cb + k, 15)];
+            pc[k] = __fmul_rn(vc[k].x, mC);
+            const float d = __fsub_rn(vc[k].x, mC);
+            ddc[k] = __fmul_rn(d, d);
+        }
+        for (int bb = b0; bb <= b1; bb += 3) {
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                if (bb + j > b1) continue;
+                const float2 vb = S.c[B][bb + j];
+                const float pb = __fmul_rn(vb.x, mB), db = __fsub_rn(vb.x, mB), ddb = __fmul_rn(db, db);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    // the test of measurement_grid.cu:88-99 (ds_is_neighbor), sums in x, y, z order; its
+                    // IEEE division is taken only where the reciprocal's result is within the rounding
+                    // of the limit
+                    const float ip = STEEP ? __fadd_rn(__fadd_rn(pb, pc[k]), pa) : __fadd_rn(__fadd_rn(pa, pb), pc[k]);
+                    const float acs = STEEP ? __fadd_rn(__fadd_rn(vb.y, vc[k].y), va.y)
+                                            : __fadd_rn(__fadd_rn(va.y, vb.y), vc[k].y);
+                    const float q = __fmul_rn(ip, ip);
+                    const float over = fmaf(-q, ex.z, acs) - wr2;
+                    bool in = over < 0.0f;
+                    if (fabsf(over) <= 3e-7f * acs) in = __fsub_rn(acs, __fdiv_rn(q, m.w)) < wr2;
+                    if (in && ip > 0.0f && cb + k <= c1) {
+                        const float r2 = STEEP ? __fadd_rn(__fadd_rn(ddb, ddc[k]), dda)  // ds_r_sqr
+                                               : __fadd_rn(__fadd_rn(dda, ddb), ddc[k]);
+                        const int li = i * stA + (bb + j) * stB + (cb + k) * stC;
+                        atomicAdd(&S.cf[li], acs > m.w ? 1u + kDsCloser : 1u);
+                        atomicMin(&S.r2[li], __float_as_uint(r2));
+                    }
+                }
+            }
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kEvThreads) k_ds_rays(EvArgs A) {
+    __shared__ ItemConst I;
+    __shared__ DsTile S;
+    __shared__ DsWarp s_warp[kEvWarps];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const unsigned lanes_below = (1u << lane) - 1u;
     const Batch& bt = A.bt;
+    const DsCells D(A);
     const uint32_t total_items = A.item_off[bt.T];
-    unsigned int* counter = COUNT ? &A.status->work_counter2 : &A.status->work_counter;
-    uint32_t* part_max = reinterpret_cast<uint32_t*>(A.acc);
-    uint32_t* part_flags = part_max + bt.C;
-    unsigned nev = 0;  // accepted neighbours of this lane (the roofline's work count, final pass)
-
+    unsigned nev = 0;  // neighbours accepted in the cells this thread finished (the roofline's work count)
     for (;;) {
-        if (threadIdx.x == 0) {
-            s_item = atomicAdd(counter, 1u);
-            s_next_sb = 0;
-        }
-        if (threadIdx.x < kRegions) s_rcnt[threadIdx.x] = 0;
+        if (wid == 0) fetch_item(A, total_items, A.chunk, &I);
         __syncthreads();
-        const uint32_t item = s_item;
-        if (item >= total_items) break;
-        const Item it = item_of(bt, A.item_off, A.tile_start, item, A.chunk);
-        if (COUNT && (it.n_items == 1 || it.k == it.n_items - 1)) {  // uniform across the block
-            __syncthreads();
-            continue;
+        if (!I.live) break;
+        const TileShape ts = I.ts;
+        const int tc[3] = {I.lt % ts.ntx, (I.lt / ts.ntx) % ts.nty, I.lt / (ts.ntx * ts.nty)};
+        const int tile_cells = ts.tx * ts.ty * ts.tz;
+        for (int i = threadIdx.x; i < tile_cells; i += kEvThreads) {
+            S.cf[i] = 0u;
+            S.r2[i] = kDsNone;
         }
-        const SceneDev& sd = bt.sc[it.sc];
-        const DevParams& p = sd.p;
-        const TileShape ts = sd.ts;
-        const FrameParams fp = bt.fp[it.sc];
-        const int coff = bt.off->cell[it.sc];
-        const int nsb = ts.nsbx * ts.nsby * (ts.tz / 2);
-        const float hres = 0.5f * p.res;
-        // Rays staged with their unit directions; in a 16x16 tile each is also listed, in input
-        // order, under the 8x8-cell columns its binned half-line (sensor -> grid exit along m)
-        // meets within the binning radius, so a sub-block visits only its column's rays, still in
-        // input order (the first-100 rule).
-        const bool regions = ts.tx == 16 && ts.ty == 16;
-        BinGeom g;
-        place_sensor(g, p, fp);
-        const float x0 = (float)(it.lt % ts.ntx * 16), y0 = (float)((it.lt / ts.ntx) % ts.nty * 16);
-        const float z0 = (float)(it.lt / (ts.ntx * ts.nty) * ts.tz);
-        const float Lc = sqrtf((float)(2 * p.G * p.G + p.Gz * p.Gz)) + 2.0f * sd.bin_R + 4.0f;  // cells
-        int step = 0;
-        for (int r0 = 0; r0 < it.nr; r0 += kEvThreads, ++step) {  // uniform trip count
-            const int r = r0 + (int)threadIdx.x;
-            unsigned qm = 0;
-            if (r < it.nr) {
-                uint32_t rid = A.evals[it.e0 + r];
-                if (rid >= (uint32_t)bt.N) rid = 0;
-                const float4 a = A.ray_a[rid];
-                sa[r] = a;
-                const float len = sqrtf(a.w);
-                const float inv = len > 0.0f ? 1.0f / len : 0.0f;
-                const float4 u = make_float4(a.x * inv, a.y * inv, a.z * inv, 0.0f);
-                su[r] = u;
-                if (regions)
-                    qm = region_mask(g.ax, g.ay, g.az, u.x * Lc, u.y * Lc, u.z * Lc, x0, y0, z0, ts.tz,
-                                     sd.bin_R + 0.25f);
+        if (threadIdx.x < 16) {
+            DevParams p;  // the fields centre_xyz reads
+            p.G = I.G; p.Gz = I.Gz; p.res = I.res;
+            const int k = threadIdx.x;
+            float x, y, z;
+            centre_xyz(tc[0] * ts.tx + k, tc[1] * ts.ty + k, tc[2] * ts.tz + k, p, I.sx, I.sy, I.sz, &x, &y, &z);
+            S.c[0][k] = make_float2(x, __fmul_rn(x, x));
+            S.c[1][k] = make_float2(y, __fmul_rn(y, y));
+            S.c[2][k] = make_float2(z, __fmul_rn(z, z));
+            if (k == 0) {
+                S.o[0] = tc[0] * ts.tx; S.o[1] = tc[1] * ts.ty; S.o[2] = tc[2] * ts.tz;
+                S.n[0] = min(ts.tx, I.G - S.o[0]); S.n[1] = min(ts.ty, I.G - S.o[1]);
+                S.n[2] = min(ts.tz, I.Gz - S.o[2]);
             }
-            if (regions) {
-                unsigned b[kRegions];
+        }
+        __syncthreads();
+        {
+            const float wr2 = bt.sc[I.sc].wr2, R = I.bin_R + 0.01f;
+            const float hg = (float)I.G / 2.0f, hz = (float)I.Gz / 2.0f;
+            const float a[3] = {I.sx / I.res + hg - 0.5f, I.sy / I.res + hg - 0.5f, I.sz / I.res + hz - 0.5f};
+            DsWarp& W = s_warp[wid];
+            for (int g = wid * 32; g < I.nr; g += kEvThreads) {
+                // one ray per lane: its line and layers; then one (ray, layer) per lane
+                int2 ly = make_int2(0, -1);
+                if (g + lane < I.nr) {
+                    uint32_t rid = A.evals[I.e0 + g + lane];
+                    if (rid >= (uint32_t)bt.N) rid = 0;  // defensive: never read past the ray arrays
+                    const float4 m = A.ray_a[rid];
+                    if (m.w > 0.0f) ly = ds_line(S, a, m, R, &W.ray[lane]);
+                }
+                const int n = max(ly.y - ly.x + 1, 0);
+                int end = n;  // inclusive prefix over the lanes
 #pragma unroll
-                for (int q = 0; q < kRegions; ++q) b[q] = __ballot_sync(0xffffffffu, (qm >> q) & 1u);
-                int(*wq)[kRegions] = s_wq[step & 1];
-                if (lane == 0) {
-#pragma unroll
-                    for (int q = 0; q < kRegions; ++q) wq[wid][q] = __popc(b[q]);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int v = __shfl_up_sync(0xffffffffu, end, o);
+                    if (lane >= o) end += v;
                 }
-                __syncthreads();
-#pragma unroll
-                for (int q = 0; q < kRegions; ++q) {
-                    if (!((qm >> q) & 1u)) continue;
-                    int pos = s_rcnt[q] + __popc(b[q] & lanes_below);
-                    for (int w = 0; w < wid; ++w) pos += wq[w][q];
-                    s_reg[q][pos] = (uint16_t)r;
+                const int total = __shfl_sync(0xffffffffu, end, 31);
+                for (int i = 0; i < n; ++i) W.layer[end - n + i] = (uint16_t)(lane | (ly.x + i) << 5);
+                __syncwarp();
+                for (int k = lane; k < total; k += 32) {
+                    const int e = W.layer[k];
+                    const DsRay& r = W.ray[e & 31];
+                    const int ax = __float_as_int(r.ext.w);
+                    if (ax == 2) ds_layer<true>(S, ts, r, 2, e >> 5, wr2);
+                    else ds_layer<false>(S, ts, r, ax, e >> 5, wr2);
                 }
-                __syncthreads();
-                if (threadIdx.x < kRegions) {
-                    int t = 0;
-                    for (int w = 0; w < kEvWarps; ++w) t += wq[w][threadIdx.x];
-                    s_rcnt[threadIdx.x] += t;
-                }
+                __syncwarp();
             }
         }
-        sb_order_keys(s_order, p, ts, it.lt, nsb, fp.sensor_x, fp.sensor_y, fp.sensor_z);
         __syncthreads();
-        sb_order_rank(s_order, nsb);
-        __syncthreads();
-        const int nr = it.nr;
-        for (;;) {
-            int sb = 0;
-            if (lane == 0) sb = atomicAdd(&s_next_sb, 1);
-            sb = __shfl_sync(0xffffffffu, sb, 0);
-            if (sb >= nsb) break;
-            sb = sb_at(s_order, sb, nsb);
-            const CellLoc L = locate(p, ts, it.lt, sb, lane, fp.sensor_x, fp.sensor_y, fp.sensor_z);
-            const float acs = __fadd_rn(__fadd_rn(__fmul_rn(L.x, L.x), __fmul_rn(L.y, L.y)), __fmul_rn(L.z, L.z));
-            int quota = kDsMaxNeighbors;
-            if (!COUNT && it.n_items > 1) {
-                int pre = 0;
-                const long base = (long)A.item_off[it.t] * kMaxTileCells;
-                for (uint32_t kk = 0; kk < it.k; ++kk) {
-                    const long idx = base + (long)kk * kMaxTileCells + L.local;
-                    pre += (idx < A.ds_count_capacity) ? (int)A.ds_counts[idx] : 0;
+        const bool single = I.n_items == 1;
+        const long base = (long)I.item * A.ds_stride;
+        for (int i = threadIdx.x; i < tile_cells; i += kEvThreads) {
+            const uint32_t cf = S.cf[i], cnt = cf & 0xFFFFu;
+            if (!single) {
+                if (base + i < A.ds_capacity) {
+                    A.ds_counts[base + i] = (uint8_t)(min(cnt, kDsMaxNeighbors + 1u) | (cf >= kDsCloser ? 0x80u : 0u));
+                    if (cnt) A.ds_r2[base + i] = S.r2[i];
                 }
-                quota = max(0, kDsMaxNeighbors - pre);
+                continue;
             }
-            if (L.c < 0) quota = 0;
-            int nb = 0;
-            bool all_far = true;
-            float mx = 0.0f;
-            const int q = sb_region(ts, sb);
-            const int nlist = regions ? s_rcnt[q] : nr;
-            if (__any_sync(0xffffffffu, quota > 0)) {
-                for (int g0 = 0; g0 < nlist; g0 += 32) {
-                    const int jl = g0 + lane;
-                    const int r = regions ? (jl < nlist ? (int)s_reg[q][jl] : 0) : jl;
-                    bool hit = false;
-                    if (jl < nlist) {
-                        // box bound on the distance from the half-line through m to the sub-block's
-                        // cell centres (the K3DOM cull's bound, with the window as the radius)
-                        const float4 u = su[r];
-                        const float qx = L.ox - hres, qy = L.oy - hres, qz = L.oz - hres;
-                        const float tproj = fmaxf(qx * u.x + qy * u.y + qz * u.z, 0.0f);
-                        const float Dx = qx - tproj * u.x, Dy = qy - tproj * u.y, Dz = qz - tproj * u.z;
-                        hit = box_reaches(Dx, Dy, Dz, Dx * Dx + Dy * Dy + Dz * Dz, hres, sd.cull_ls2);
-                    }
-                    // candidates in input order (the first-100 rule counts them in that order)
-                    const unsigned mask = __ballot_sync(0xffffffffu, hit);
-                    if (hit) s_cand[wid][__popc(mask & lanes_below)] = (uint16_t)r;
-                    __syncwarp();
-                    const int ncand = __popc(mask);
-                    for (int k = 0; k < ncand; ++k) {
-                        const float4 a = sa[s_cand[wid][k]];
-                        if (nb < quota && ds_is_neighbor(L.x, L.y, L.z, acs, a, sd.wr2)) {
-                            ++nb;
-                            if (!COUNT) {
-                                ++nev;
-                                if (acs > a.w) all_far = false;
-                                const float o = ds_pocc(L.x, L.y, L.z, a, p.meas_occ_stddev);
-                                if (o > mx) mx = o;
-                            }
-                        }
-                    }
-                    __syncwarp();
-                    if (!__any_sync(0xffffffffu, nb < quota)) break;
-                }
+            if (!cnt) continue;
+            const int lx = i % ts.tx, ly = (i / ts.tx) % ts.ty, lz = i / (ts.tx * ts.ty);
+            const int c = I.coff + (S.o[0] + lx) + I.G * (S.o[1] + ly) + I.G * I.G * (S.o[2] + lz);
+            nev += min(cnt, kDsMaxNeighbors);
+            if (cnt <= kDsMaxNeighbors) {
+                D.r2[c] = S.r2[i];
+                D.flags[c] = 1u | (cf >= kDsCloser ? 2u : 0u);
+            } else {
+                const uint32_t w = atomicAdd(&A.status->work_counter2, 1u);
+                D.work_cell[w] = (uint32_t)c;
+                D.work_item[w] = I.item;
             }
-            if (COUNT) {
-                if (L.c >= 0) {
-                    const long idx = (long)item * kMaxTileCells + L.local;
-                    if (idx < A.ds_count_capacity) A.ds_counts[idx] = (uint8_t)nb;
-                }
-            } else if (L.c >= 0 && nb > 0) {
-                const int c = coff + L.c;
-                atomicMax(&part_max[c], __float_as_uint(mx));
-                atomicOr(&part_flags[c], 1u | (all_far ? 0u : 2u));
-            }
-        }
-        if (COUNT) {
-            __syncthreads();
-            continue;
-        }
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) s_last = (atomicAdd(&A.tile_done[it.t], 1u) == it.n_items - 1) ? 1 : 0;
-        __syncthreads();
-        if (s_last) {
-            __threadfence();
-            const int tx = it.lt % ts.ntx, ty = (it.lt / ts.ntx) % ts.nty, tz = it.lt / (ts.ntx * ts.nty);
-            const int tile_cells = ts.tx * ts.ty * ts.tz;
-            for (int li = threadIdx.x; li < tile_cells; li += kEvThreads) {
-                const int lx = li % ts.tx, ly = (li / ts.tx) % ts.ty, lz = li / (ts.tx * ts.ty);
-                const int ix = tx * ts.tx + lx, iy = ty * ts.ty + ly, iz = tz * ts.tz + lz;
-                if (ix >= p.G || iy >= p.G || iz >= p.Gz) continue;
-                const int c = coff + ix + p.G * iy + p.G * p.G * iz;
-                const uint32_t m = __ldcg(&part_max[c]);
-                const uint32_t f = __ldcg(&part_flags[c]);
-                if (m) __stcg(&part_max[c], 0u);
-                if (f) __stcg(&part_flags[c], 0u);
-                float x, y, z;
-                centre_xyz(ix, iy, iz, p, fp.sensor_x, fp.sensor_y, fp.sensor_z, &x, &y, &z);
-                const float acs = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
-                const DsMeas mc = ds_meas_from(p, acs, (f & 1u) ? 1 : 0, (f & 2u) == 0, __uint_as_float(m));
-                ds_cell_update(p, c, mc, A.cs, A.cw, A.first_frame != 0);
-            }
-            if (threadIdx.x == 0) A.tile_done[it.t] = 0;
         }
         __syncthreads();
     }
-    if (!COUNT) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) nev += __shfl_xor_sync(0xffffffffu, nev, o);
-        if (lane == 0 && nev) atomicAdd(&A.status->kernel_evals, (unsigned long long)nev);
+    for (int o = 16; o > 0; o >>= 1) nev += __shfl_xor_sync(0xffffffffu, nev, o);
+    if (lane == 0 && nev) atomicAdd(&A.status->kernel_evals, (unsigned long long)nev);
+}
+
+// The tiles with several items, a cell per thread and kEvThreads cells per CTA.
+__global__ void __launch_bounds__(kEvThreads) k_ds_combine(EvArgs A, int ctas_per_tile) {
+    const Batch& bt = A.bt;
+    const DsCells D(A);
+    const int t = blockIdx.x / ctas_per_tile, i = (blockIdx.x % ctas_per_tile) * kEvThreads + threadIdx.x;
+    const uint32_t first = A.item_off[t], n_items = A.item_off[t + 1] - first;
+    if (n_items <= 1) return;
+    const int sc = scene_of(bt.off->tile, bt.S, t);
+    const SceneDev& sd = bt.sc[sc];
+    const TileShape ts = sd.ts;
+    const int lt = t - bt.off->tile[sc], G = sd.p.G, Gz = sd.p.Gz;
+    const int ix = lt % ts.ntx * ts.tx + i % ts.tx, iy = (lt / ts.ntx) % ts.nty * ts.ty + (i / ts.tx) % ts.ty;
+    const int iz = lt / (ts.ntx * ts.nty) * ts.tz + i / (ts.tx * ts.ty);
+    unsigned nev = 0;
+    if (i < ts.tx * ts.ty * ts.tz && ix < G && iy < G && iz < Gz) {
+        const int c = bt.off->cell[sc] + ix + G * iy + G * G * iz;
+        uint32_t pre = 0, r2 = kDsNone, closer = 0;
+        constexpr uint32_t kAhead = 8;  // counts read at once: a tile next to the sensor has many items
+        bool open = true;
+        for (uint32_t k0 = 0; k0 < n_items && open; k0 += kAhead) {
+            uint32_t cf[kAhead];
+#pragma unroll
+            for (uint32_t j = 0; j < kAhead; ++j) {
+                const long e = (long)(first + k0 + j) * A.ds_stride + i;
+                cf[j] = k0 + j < n_items && e < A.ds_capacity ? A.ds_counts[e] : 0u;
+            }
+#pragma unroll
+            for (uint32_t j = 0; j < kAhead; ++j) {
+                const uint32_t cnt = cf[j] & 0x7Fu;
+                if (!cnt || !open) continue;
+                if (pre + cnt > kDsMaxNeighbors) {
+                    open = false;
+                    if (pre < kDsMaxNeighbors) {  // the item that holds the hundredth neighbour
+                        const uint32_t w = atomicAdd(&A.status->work_counter2, 1u);
+                        D.work_cell[w] = (uint32_t)c;
+                        D.work_item[w] = first + k0 + j;
+                        nev += kDsMaxNeighbors - pre;
+                    }
+                    continue;
+                }
+                pre += cnt;
+                closer |= cf[j] & 0x80u;
+                r2 = min(r2, A.ds_r2[(long)(first + k0 + j) * A.ds_stride + i]);
+            }
+        }
+        if (pre) {
+            nev += pre;
+            D.r2[c] = r2;
+            D.flags[c] = 1u | (closer ? 2u : 0u);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) nev += __shfl_xor_sync(0xffffffffu, nev, o);
+    if ((threadIdx.x & 31) == 0 && nev) atomicAdd(&A.status->kernel_evals, (unsigned long long)nev);
+}
+
+// A warp per worklist entry: the first (100 - neighbours of the tile's earlier items) neighbours of
+// the cell among the item's rays, in list order, added to the cell's result.
+__global__ void __launch_bounds__(kEvThreads) k_ds_partial(EvArgs A) {
+    const Batch& bt = A.bt;
+    const DsCells D(A);
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    const uint32_t n = A.status->work_counter2;
+    for (uint32_t w = blockIdx.x * kEvWarps + (threadIdx.x >> 5); w < n; w += gridDim.x * kEvWarps) {
+        const int c = (int)D.work_cell[w];
+        const uint32_t item = D.work_item[w];
+        const int t = warp_find_tile(A.item_off, bt.T, item);
+        const int sc = scene_of(bt.off->cell, bt.S, c);
+        const SceneDev& sd = bt.sc[sc];
+        const FrameParams& fp = bt.fp[sc];
+        const TileShape ts = sd.ts;
+        int ix, iy, iz;
+        cell_xyz(c - bt.off->cell[sc], sd.p.G, &ix, &iy, &iz);
+        const int li = ix % ts.tx + ts.tx * (iy % ts.ty + ts.ty * (iz % ts.tz));
+        const uint32_t first = A.item_off[t];
+        int quota = (int)kDsMaxNeighbors;
+        for (uint32_t k = first; k < item; k += 32) {
+            const long e = (long)(k + lane) * A.ds_stride + li;
+            const int cnt = k + lane < item && e < A.ds_capacity ? A.ds_counts[e] & 0x7F : 0;
+            quota -= (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+        }
+        float x, y, z;
+        centre_xyz(ix, iy, iz, sd.p, fp.sensor_x, fp.sensor_y, fp.sensor_z, &x, &y, &z);
+        const float acs = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
+        const uint32_t e0 = A.tile_start[t] + (item - first) * (uint32_t)A.chunk;
+        const uint32_t e1 = min(A.tile_start[t + 1], e0 + (uint32_t)A.chunk);
+        uint32_t r2 = kDsNone, closer = 0;
+        for (uint32_t e = e0; e < e1 && quota > 0; e += 32) {
+            bool in = false;
+            float4 m = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (e + lane < e1) {
+                uint32_t rid = A.evals[e + lane];
+                if (rid >= (uint32_t)bt.N) rid = 0;
+                m = A.ray_a[rid];
+                in = ds_is_neighbor(x, y, z, acs, m, sd.wr2);
+            }
+            const unsigned mask = __ballot_sync(0xffffffffu, in);
+            if (in && __popc(mask & below) < quota) {
+                r2 = min(r2, __float_as_uint(ds_r_sqr(x, y, z, m)));
+                if (acs > m.w) closer = 2u;
+            }
+            quota -= __popc(mask);
+        }
+        r2 = __reduce_min_sync(0xffffffffu, r2);
+        closer = __reduce_or_sync(0xffffffffu, closer);
+        if (lane == 0) {
+            const uint32_t f = D.flags[c];
+            D.r2[c] = (f & 1u) ? min(D.r2[c], r2) : r2;
+            D.flags[c] = f | 1u | closer;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kBlock) k_ds_update(EvArgs A) {
+    const Batch& bt = A.bt;
+    const DsCells D(A);
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < bt.C; c += gridDim.x * blockDim.x) {
+        const int sc = scene_of(bt.off->cell, bt.S, c);
+        const SceneDev& sd = bt.sc[sc];
+        const FrameParams& fp = bt.fp[sc];
+        const uint32_t f = D.flags[c];
+        float acs = 0.0f, occ = 0.0f;
+        if (f) {
+            D.flags[c] = 0u;
+            int ix, iy, iz;
+            cell_xyz(c - bt.off->cell[sc], sd.p.G, &ix, &iy, &iz);
+            float x, y, z;
+            centre_xyz(ix, iy, iz, sd.p, fp.sensor_x, fp.sensor_y, fp.sensor_z, &x, &y, &z);
+            acs = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
+            occ = ds_pocc(__uint_as_float(D.r2[c]), sd.p.meas_occ_stddev);
+        }
+        const DsMeas mc = ds_meas_from(sd.p, acs, (f & 1u) ? 1 : 0, (f & 2u) == 0, occ);
+        ds_cell_update(sd.p, c, mc, A.cs, A.cw, A.first_frame != 0);
     }
 }
 
@@ -2028,8 +2162,10 @@ static EvArgs make_args(const Batch& bt, RayBuffers& rb, CellState cs, CellWork 
     A.item_slots = rb.item_slots;
     A.tile_done = rb.tile_done;
     A.acc = rb.acc;
+    A.ds_r2 = rb.ds_r2;
     A.ds_counts = rb.ds_counts;
-    A.ds_count_capacity = rb.ds_count_capacity;
+    A.ds_capacity = rb.ds_capacity;
+    A.ds_stride = rb.ds_stride;
     A.cs = cs;
     A.cw = cw;
     A.status = status;
@@ -2361,40 +2497,38 @@ cudaError_t launch_k3dom_update_cells(const Batch& bt, RayBuffers& rb, CellState
     return cudaGetLastError();
 }
 
-// The DS launches are persistent too: the count pass and the final pass each get one CTA per
-// resident slot (the count pass fits 5 CTAs per SM at 47 registers, the final pass 4).
-struct DsLaunch {
-    int count_blocks, final_blocks;
-};
-
-static DsLaunch ds_launch() {
-    int dev = 0, sms = 148, per_count = 1, per_final = 1;
+// The DS passes: k_ds_rays is persistent, one CTA per resident slot; k_ds_partial gets as many.
+static int ds_blocks(const void* kern) {
+    int dev = 0, sms = 148, per = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_count, k_dsgrid<true>, kEvThreads, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_final, k_dsgrid<false>, kEvThreads, 0);
-    return DsLaunch{sms * std::max(1, per_count), sms * std::max(1, per_final)};
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kEvThreads, 0);
+    return sms * std::max(1, per);
 }
 
-void k3dom_ds_evidence_blocks(int* count_blocks, int* final_blocks) {
-    const DsLaunch L = ds_launch();
-    *count_blocks = L.count_blocks;
-    *final_blocks = L.final_blocks;
+void k3dom_ds_evidence_blocks(int* ray_blocks, int* partial_blocks) {
+    *ray_blocks = ds_blocks((const void*)k_ds_rays);
+    *partial_blocks = ds_blocks((const void*)k_ds_partial);
 }
 
-cudaError_t launch_ds_evidence(const Batch& bt, RayBuffers& rb, CellState cs, CellWork cw, bool first_frame,
-                               DevStatus* status, cudaStream_t st) {
+cudaError_t launch_ds_measure(const Batch& bt, RayBuffers& rb, DevStatus* status, cudaStream_t st) {
     if (rb.chunk < 32 || rb.chunk > kChunk) return cudaErrorInvalidValue;
-    EvArgs A = make_args(bt, rb, cs, cw, first_frame, status);
-    const DsLaunch L = ds_launch();
-    ++g_launches;
-    k_dsgrid<true><<<L.count_blocks, kEvThreads, 0, st>>>(A);
-    ++g_launches;
-    k_dsgrid<false><<<L.final_blocks, kEvThreads, 0, st>>>(A);
+    const EvArgs A = make_args(bt, rb, CellState{}, CellWork{}, false, status);
+    g_launches += 3;
+    k_ds_rays<<<ds_blocks((const void*)k_ds_rays), kEvThreads, 0, st>>>(A);
+    const int per_tile = div_up(rb.ds_stride, kEvThreads);
+    k_ds_combine<<<bt.T * per_tile, kEvThreads, 0, st>>>(A, per_tile);
+    k_ds_partial<<<ds_blocks((const void*)k_ds_partial), kEvThreads, 0, st>>>(A);
     return cudaGetLastError();
 }
 
-long ds_count_bytes(long items) { return items * (long)kMaxTileCells; }
+cudaError_t launch_ds_update(const Batch& bt, RayBuffers& rb, CellState cs, CellWork cw, bool first_frame,
+                             DevStatus* status, cudaStream_t st) {
+    const EvArgs A = make_args(bt, rb, cs, cw, first_frame, status);
+    ++g_launches;
+    k_ds_update<<<div_up(bt.C, kBlock), kBlock, 0, st>>>(A);
+    return cudaGetLastError();
+}
 
 cudaError_t evidence_init() {
     cudaError_t e = cudaFuncSetAttribute(k_bgki, cudaFuncAttributeMaxDynamicSharedMemorySize,

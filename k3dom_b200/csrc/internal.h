@@ -147,14 +147,16 @@ struct RayBuffers {
     uint32_t* item_off;    // T+1 work-item offsets per tile
     uint32_t* tile_done;   // T
     unsigned long long* acc;  // 2*C fixed-point accumulators (K3DOM) / DS partials
-    uint8_t* ds_counts;    // DS: per (item, cell) neighbour counts of pass 1
+    uint32_t* ds_r2;       // DS: per (item, cell) smallest squared point distance (float bits)
+    uint8_t* ds_counts;    // DS: per (item, cell) neighbours (101 = more than 100), bit 7: one closer than the cell
     uint32_t* scan_tmp;
     long scan_words;
     uint32_t* os_scratch;  // onesweep sort of the entries by tile
     long os_words;
     uint32_t* total;       // [0] = entries, [2] = entries kept (0 on overflow)
     long capacity;         // entries
-    long ds_count_capacity;
+    long ds_capacity;      // DS: (item, cell) summaries
+    int ds_stride;         // DS: cells of the largest tile
     int chunk;             // largest number of rays per work item
     int item_slots;        // CTA slots the work items are spread over (0: items of chunk rays whatever the scene)
 };
@@ -178,15 +180,16 @@ cudaError_t launch_k3dom_evidence(const Batch& bt, RayBuffers& rb, CellState cs,
 // The cell update of a K3DOM frame whose evidence ran with fuse_update = false.
 cudaError_t launch_k3dom_update_cells(const Batch& bt, RayBuffers& rb, CellState cs, CellWork cw, DevStatus* status,
                                       cudaStream_t st);
-cudaError_t launch_ds_evidence(const Batch& bt, RayBuffers& rb, CellState cs, CellWork cw, bool first_frame,
-                               DevStatus* status, cudaStream_t st);
+// DS: the measurement grid from the ray lists, then the masses of every cell.
+cudaError_t launch_ds_measure(const Batch& bt, RayBuffers& rb, DevStatus* status, cudaStream_t st);
+cudaError_t launch_ds_update(const Batch& bt, RayBuffers& rb, CellState cs, CellWork cw, bool first_frame,
+                             DevStatus* status, cudaStream_t st);
 // CTA slots of the K3DOM and calibration evidence kernels, for RayBuffers::item_slots.
 int evidence_slots(int num_sms);
 // CTAs of the K3DOM evidence launch for a chunk size (persistent grid).
 int k3dom_evidence_blocks(int chunk);
-// CTAs of the DS count pass and final pass (persistent: one per resident slot of each build).
-void k3dom_ds_evidence_blocks(int* count_blocks, int* final_blocks);
-long ds_count_bytes(long items);
+// CTAs of the DS pass over the rays and of the pass over the cells past 100 neighbours.
+void k3dom_ds_evidence_blocks(int* ray_blocks, int* partial_blocks);
 cudaError_t evidence_init();
 // Host: the sparse-kernel table for sigma, every value multiplied by scale: 512 intervals and a
 // zero entry at u = 1 (513 float4), so an index taken at the support's edge needs no clamp.
