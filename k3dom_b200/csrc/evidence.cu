@@ -207,7 +207,12 @@ __device__ __forceinline__ RayPrep prep_ray(const DevParams& p, const BinGeom& g
             r.ok = false;  // |m| = 0: inner product 0, never a neighbour (measurement_grid.cu:92)
             return r;
         }
-        const float L = sqrtf((float)(2 * g.G * g.G + g.Gz * g.Gz)) + 2.0f * g.R + 4.0f;  // cells
+        // length of the binned half-line in cells: past the grid's far corner, also from a sensor
+        // outside the grid
+        const float diag = sqrtf((float)(2 * g.G * g.G + g.Gz * g.Gz));
+        const float cx = g.ax - 0.5f * (float)(g.G - 1), cy = g.ay - 0.5f * (float)(g.G - 1);
+        const float cz = g.az - 0.5f * (float)(g.Gz - 1);
+        const float L = fmaxf(diag, 0.5f * diag + sqrtf(cx * cx + cy * cy + cz * cz)) + 2.0f * g.R + 4.0f;
         const float sc = L / (len / p.res);
         r.bx = g.ax + mx / p.res * sc;
         r.by = g.ay + my / p.res * sc;

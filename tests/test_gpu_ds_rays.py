@@ -47,7 +47,7 @@ def rays(kind, n, reach, seed):
     (33, 9, 0.2, "scan", 1, (0, 0, 0)), (33, 9, 0.2, "scan", 33, (0, 0, 0)), (33, 9, 0.2, "scan", 6000, (0.13, -0.4, 0.2)),
     (40, 12, 0.1, "steep", 3000, (0, 0, 0)), (36, 11, 0.1, "axis", 300, (0.05, 0.05, 0.05)),
     (50, 10, 0.1, "bundle", 2500, (-1.0, 0.2, 0.0)), (24, 10, 0.4, "bundle", 700, (0, 0, 0)),
-    (20, 6, 0.1, "scan", 4000, (0, 0, 0)),
+    (20, 6, 0.1, "scan", 4000, (0, 0, 0)), (47, 17, 0.1, "scan", 20000, (3.0, -4.0, 0.3)),
 ])
 def test_measurement_matches_oracle(G, Gz, res, kind, n, sensor):
     from oracle import binding as O
