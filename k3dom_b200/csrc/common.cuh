@@ -39,8 +39,7 @@ struct SceneDev {
     TileShape ts;
     int cell_off, part_off, birth_off, joint_off, point_off, tile_off;
     int n_tiles, max_points;
-    float bin_R;    // ray-binning support radius [cells]
-    float cull_r2;   // DS: squared cull radius around a sub-block centroid [m^2]
+    float bin_R;    // ray-binning support radius [cells] (DS: an upper bound, see ds_window)
     float wr2;       // DS window radius squared [m^2]
     float cull_ls2;  // K3DOM: squared support radius of the sub-block cull, ls plus slack [m^2]
     double fx_inv;   // K3DOM evidence: value = fixed-point integer * fx_inv

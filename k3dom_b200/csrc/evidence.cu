@@ -222,9 +222,23 @@ __device__ __forceinline__ RayPrep prep_ray(const DevParams& p, const BinGeom& g
 }
 
 
+// The distance from a ray's half-line within which a cell can pass the DS neighbour test, in cells, for
+// cells at most `dist` metres from the sensor. The test compares |c|^2 - (c.m)^2 / |m|^2 with the
+// window in FP32: the two terms carry at most 3 and 11 roundings of |c|^2, 8.4e-7 of it together.
+__device__ __forceinline__ float ds_window(float wr2, float dist2, float res) {
+    return sqrtf(wr2 + 1e-6f * dist2) / res + 1e-3f;
+}
+// (A slack for cells up to twice the grid's extent away made the window 2.05 cells at 256 cells of
+// 0.1 m instead of 0.9: 120,000 rays, lists 158 -> 139 us, k_ds_rays 0.62 -> 0.18 ms.)
+
 __device__ __forceinline__ BinGeom scene_geom(const SceneDev& sd, const FrameParams& f) {
     BinGeom g;
     g.R = sd.bin_R;
+    if (sd.p.variant != 0) {  // DS: from the farthest cell
+        const float ext = sqrtf(f.sensor_x * f.sensor_x + f.sensor_y * f.sensor_y + f.sensor_z * f.sensor_z) +
+                          0.5f * sd.p.res * sqrtf((float)(2 * sd.p.G * sd.p.G + sd.p.Gz * sd.p.Gz));
+        g.R = fminf(g.R, ds_window(sd.wr2, ext * ext, sd.p.res) + 0.02f);  // 0.02: the tile walk's arithmetic
+    }
     g.G = sd.p.G;
     g.Gz = sd.p.Gz;
     g.tx = sd.ts.tx; g.ty = sd.ts.ty; g.tz = sd.ts.tz;
@@ -507,33 +521,14 @@ void fill_scene_evidence(SceneDev& sd, bool ds, float4* ktab) {
     if (!ds) {
         sd.bin_R = p.ls / p.res * (1.0f + 1e-4f) + 1e-3f;
     } else {
-        // window radius plus the FP32 rounding slack of |c|^2 - (c.m)^2/|m|^2
+        // an upper bound of ds_window's radius, for the capacity of the ray lists
         const float ext = max_extent(p);
         const float slack = 64.0f * 5.96e-8f * ext * ext;
         sd.bin_R = sqrtf(p.window_radius * p.window_radius + slack) / p.res + 1e-3f;
     }
     sd.wr2 = p.window_radius * p.window_radius;
-    // cull around the sub-block centroid: half diagonal sqrt(1.5^2+1.5^2+0.5^2) res
-    const float rsb = 2.1794495f * p.res;
-    float rsup;
-    if (!ds) {
-        rsup = p.ls * (1.0f + 1e-4f) + rsb + 1e-3f * p.res;
-    } else {
-        const float ext = max_extent(p);
-        const float slack = 64.0f * 5.96e-8f * ext * ext;
-        rsup = sqrtf(p.window_radius * p.window_radius + slack) + rsb + 1e-3f * p.res;
-    }
-    sd.cull_r2 = rsup * rsup;
-    // box culls (stage_pair, k_dsgrid): the support radius, or the DS window with the FP32 slack
-    // of the reference's neighbour test, plus the same margin as rsup
-    float rls;
-    if (!ds) {
-        rls = p.ls * (1.0f + 1e-4f) + 1e-3f * p.res;
-    } else {
-        const float ext = max_extent(p);
-        const float slack = 64.0f * 5.96e-8f * ext * ext;
-        rls = sqrtf(p.window_radius * p.window_radius + slack) + 1e-3f * p.res;
-    }
+    // K3DOM box culls (box_reaches): the support radius with a margin
+    const float rls = p.ls * (1.0f + 1e-4f) + 1e-3f * p.res;
     sd.cull_ls2 = rls * rls;
     // fixed point: the table is scaled by a power of two so that a kernel value is at most 1, and
     // one unit is 2^-40 of that: at most 2^40 units a value, leaving 2^23 terms of headroom in a
@@ -1780,12 +1775,12 @@ __device__ __forceinline__ float ds_pocc(float r_sqr, float delta) {
 //   k_ds_combine  cells of tiles with several items: the items in order up to the hundredth neighbour
 //   k_ds_partial  the worklist
 //   k_ds_update   the measurement-to-mass step and the Dempster update of every cell
-// 256x256x32 voxels at 0.1 m, 120,000 rays: the lane-per-cell passes took 0.65 + 1.10 ms, these 0.62 +
-// 0.07 + 0.04 + 0.05 ms; 200x200x25 at 0.2 m, 60,000 rays: 0.69 -> 0.33 ms. k_ds_rays is bound by
-// instruction issue and by its waits at the items' ends (1,560 thread instructions per (tile, ray)
-// entry; 20 of 32 lanes in the layers' loops). One ray per lane with the layers as a loop ran at 6 of
-// 32 lanes (1.52 ms), one (ray, layer) per lane with plain loops over its cells 0.86 ms; CTAs of 128
-// or 64 threads wait less but leave longer tails (0.87 and 1.10 ms).
+// 256x256x32 voxels at 0.1 m, 120,000 rays: the lane-per-cell passes took 0.65 + 1.10 ms, these 0.18 +
+// 0.04 + 0.07 + 0.05 ms; 200x200x25 at 0.2 m, 60,000 rays: 0.69 -> 0.20 ms. k_ds_rays is bound by
+// instruction issue and by its waits at the items' ends. With the window of the lists at 2.05 cells
+// (see ds_window): one ray per lane with the layers as a loop ran at 6 of 32 lanes (1.52 ms), one
+// (ray, layer) per lane with plain loops over its cells 0.86 ms, with unrolled blocks 0.62 ms; CTAs of
+// 128 or 64 threads wait less but leave longer tails (1.01x and 1.27x the time).
 constexpr int kMaxTileCells = 16 * 16 * 8;
 constexpr uint32_t kDsNone = 0xFFFFFFFFu;
 constexpr uint32_t kDsCloser = 0x10000u;  // in a cell's counter: neighbours | closer ones << 16
@@ -1951,7 +1946,12 @@ __global__ void __launch_bounds__(kEvThreads) k_ds_rays(EvArgs A) {
         }
         __syncthreads();
         {
-            const float wr2 = bt.sc[I.sc].wr2, R = I.bin_R + 0.01f;
+            const float wr2 = bt.sc[I.sc].wr2;
+            // the window at the tile's farthest cell, and 0.01 cells for the walk's own arithmetic
+            float far2 = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) far2 += fmaxf(S.c[k][0].y, S.c[k][S.n[k] - 1].y);
+            const float R = ds_window(wr2, far2, I.res) + 0.01f;
             const float hg = (float)I.G / 2.0f, hz = (float)I.Gz / 2.0f;
             const float a[3] = {I.sx / I.res + hg - 0.5f, I.sy / I.res + hg - 0.5f, I.sz / I.res + hz - 0.5f};
             DsWarp& W = s_warp[wid];
