@@ -116,8 +116,11 @@ __device__ __forceinline__ void view_cell(const DevParams& p, int c, CellState c
 
 __device__ __forceinline__ float total_mass(const CellView& v) { return __fadd_rn(__fadd_rn(v.f, v.s), v.d); }
 
-__global__ void k_export_field(DevParams p, int field, CellState cs, CellWork cw, const float* born_cum,
-                               int range_base, float* dst) {
+// One build per field: each reads only the arrays its field needs (all of them, 80 bytes a cell, took
+// 25 us and more beside the births of a 2.1 M-cell frame).
+template <int field>
+__global__ void k_export_field(DevParams p, CellState cs, CellWork cw, const float* born_cum, int range_base,
+                               float* dst) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= p.C) return;
     CellView v;
@@ -164,7 +167,36 @@ __global__ void k_export_field(DevParams p, int field, CellState cs, CellWork cw
 void launch_export_field(const DevParams& p, int field, CellState cs, CellWork cw, const float* born_cum,
                          int range_base, float* dst, cudaStream_t st) {
     ++g_launches;
-    k_export_field<<<div_up(p.C, kBlock), kBlock, 0, st>>>(p, field, cs, cw, born_cum, range_base, dst);
+    const int blocks = div_up(p.C, kBlock);
+    auto run = [&](auto kern) { kern<<<blocks, kBlock, 0, st>>>(p, cs, cw, born_cum, range_base, dst); };
+    switch (field) {
+        case 0: run(k_export_field<0>); break;
+        case 1: run(k_export_field<1>); break;
+        case 2: run(k_export_field<2>); break;
+        case 3: run(k_export_field<3>); break;
+        case 4: run(k_export_field<4>); break;
+        case 5: run(k_export_field<5>); break;
+        case 6: run(k_export_field<6>); break;
+        case 7: run(k_export_field<7>); break;
+        case 8: run(k_export_field<8>); break;
+        case 9: run(k_export_field<9>); break;
+        case 10: run(k_export_field<10>); break;
+        case 11: run(k_export_field<11>); break;
+        case 12: run(k_export_field<12>); break;
+        case 13: run(k_export_field<13>); break;
+        case 14: run(k_export_field<14>); break;
+        case 15: run(k_export_field<15>); break;
+        case 16: run(k_export_field<16>); break;
+        case 17: run(k_export_field<17>); break;
+        case 18: run(k_export_field<18>); break;
+        case 19: run(k_export_field<19>); break;
+        case 20: run(k_export_field<20>); break;
+        case 21: run(k_export_field<21>); break;
+        case 22: run(k_export_field<22>); break;
+        case 23: run(k_export_field<23>); break;
+        case 24: run(k_export_field<24>); break;
+        default: run(k_export_field<-1>);
+    }
 }
 
 // dom::GridCell, include/common/dom_types.h:12-45 (68 bytes).
