@@ -53,6 +53,7 @@ struct SceneOffsets {
     int cell[kMaxScenes + 1];
     int point[kMaxScenes + 1];
     int tile[kMaxScenes + 1];
+    int draw[kMaxScenes + 1];  // blocks of the draws' passes (draw_blocks of each scene)
 };
 
 // Per-frame scalars, resident in device memory so a captured graph can be replayed.

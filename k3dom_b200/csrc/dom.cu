@@ -140,9 +140,8 @@ struct k3dom_handle {
     void* exact_scratch = nullptr;
     ExactTile *plan_born = nullptr, *plan_joint = nullptr;
     int plan_born_n = 0, plan_joint_n = 0;
-    uint32_t *draw_keys = nullptr, *draw_sorted = nullptr, *draw_alt = nullptr;
-    uint32_t* os_draw = nullptr;  // onesweep scratch of the draw sort (runs on the second stream)
-    long os_draw_words = 0;
+    uint32_t* draw_sorted = nullptr;
+    DrawScratch draw_scratch{};
     cudaEvent_t ev_staged = nullptr;  // host staging (frame scalars, points) consumed
     int* ancestors = nullptr;
     float* pts = nullptr;  // device x | y | z, N slots each
@@ -740,11 +739,8 @@ cudaError_t enq_births(k3dom_handle* h) {
 }
 
 cudaError_t enq_draws(k3dom_handle* h, cudaStream_t s) {
-    launch_draw_keys(h->batch(), h->draw_keys, s);
-    SortWait w = h->sort_wait;
-    w.skip_tile = -1;
-    return onesweep_sort_pairs(h->draw_keys, nullptr, h->draw_sorted, nullptr, h->draw_alt, nullptr, h->P,
-                               draw_key_bits(h->S), h->os_draw, h->os_draw_words, h->status, w, s);
+    launch_sorted_draws(h->batch(), h->off.draw[h->S], h->draw_scratch, h->draw_sorted, s);
+    return cudaGetLastError();
 }
 
 cudaError_t enq_resample(k3dom_handle* h, bool draws_ready) {
@@ -977,6 +973,7 @@ k3dom_status k3dom_batch_create(const k3dom_params* params, int32_t n_scenes, k3
         h->off.birth[s] = B;
         h->off.joint[s] = P + B;
         h->off.cell[s] = C;
+        h->off.draw[s + 1] = h->off.draw[s] + draw_blocks(x.dp.P);
         P += x.dp.P;
         B += x.dp.B;
         C += x.dp.C;
@@ -1060,14 +1057,13 @@ k3dom_status k3dom_batch_create(const k3dom_params* params, int32_t n_scenes, k3
         if ((e = h->alloc(&es, sb))) return bail(e);
         h->exact_scratch = es;
     }
-    if ((e = h->alloc(&h->draw_keys, P)) || (e = h->alloc(&h->draw_sorted, P)) || (e = h->alloc(&h->draw_alt, P)))
+    if ((e = h->alloc(&h->draw_sorted, P)) || (e = h->alloc(&h->draw_scratch.totals, draw_bucket_words(h->S))) ||
+        (e = h->alloc(&h->draw_scratch.starts, draw_bucket_words(h->S))) ||
+        (e = h->alloc(&h->draw_scratch.keys, P)) || (e = h->alloc(&h->draw_scratch.rows, draw_row_words(h->off.draw[h->S]))))
         return bail(e);
-    // sort scratch of the particle sort, and a separate one for the draw sort (it runs
-    // concurrently on the second stream; the draw keys carry the scene index above 24 bits)
+    // scratch of the particle sort
     h->os_words = onesweep_scratch_words(P, key_bits_for(h->C));
     if ((e = h->alloc(&h->os_scratch, h->os_words))) return bail(e);
-    h->os_draw_words = onesweep_scratch_words(P, draw_key_bits(h->S));
-    if ((e = h->alloc(&h->os_draw, h->os_draw_words))) return bail(e);
     if ((e = alloc_ray_buffers(h))) return bail(e);
     // DOM_c::initialize (src/common/dom.cu:90-109): cells to priors
     launch_cells_init(h->batch(), h->cs[0], h->cw, h->st);

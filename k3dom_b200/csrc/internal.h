@@ -102,14 +102,23 @@ void launch_gather_segsum(const Batch& bt, const float4* x, Particles s, const u
 void launch_reweight(const Batch& bt, Particles s, const uint32_t* sorted_keys, CellWork cw, cudaStream_t st);
 void launch_births(const Batch& bt, const float* born, const float* born_cum, Particles b, cudaStream_t st);
 void launch_init_particles(const Batch& bt, const float* born_cum, Particles a, cudaStream_t st);
-int draw_key_bits(int S);
-void launch_draw_keys(const Batch& bt, uint32_t* keys, cudaStream_t st);
 long res_bracket_count(long P);
 void launch_resample(const Batch& bt, const float* joint_cum, const uint32_t* sorted_draws, Particles s,
                      Particles b, Particles out, int* ancestors, float* joint_max_out, int2* brackets,
                      cudaStream_t st);
 void launch_debug_draws(uint64_t seed, int frame, int stage, long first, long count, float* dst,
                         cudaStream_t st);
+
+// drawsort.cu: the frame's resampling draws as 24-bit keys of 1 - u, sorted within each scene's
+// particle range.
+constexpr int kDrawPerBlock = 16384;
+int draw_blocks(int P);              // blocks of a scene of P particles
+long draw_row_words(int blocks);     // words of DrawScratch::rows
+long draw_bucket_words(int S);       // words of totals and of starts
+struct DrawScratch {
+    uint32_t *totals, *starts, *rows, *keys;  // totals: zero between calls; keys: one per particle
+};
+void launch_sorted_draws(const Batch& bt, int blocks, const DrawScratch& d, uint32_t* sorted, cudaStream_t st);
 
 // cells.cu
 void launch_cells_init(const Batch& bt, CellState cs, CellWork cw, cudaStream_t st);

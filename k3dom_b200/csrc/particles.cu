@@ -521,32 +521,6 @@ void launch_init_particles(const Batch& bt, const float* born_cum, Particles a, 
 }
 
 // ---------------------------------------------------------------- resampling
-// Resampling draws as 24-bit keys of 1 - u: sorting the keys ascending orders the draws
-// u * joint_max ascending for any joint_max >= 0, so the draws can be sorted before the
-// weights exist (resamplingGenerateRandomNumbersKernel + thrust::sort, resampling.cu:38-53,
-// src/common/dom.cu:277-285). The scene index sits above the 24 key bits, so one sort orders
-// every scene's draws within the scene's own particle range.
-__global__ void k_draw_keys(Batch bt, uint32_t* keys) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < bt.P; i += gridDim.x * blockDim.x) {
-        const int sc = scene_of(bt.off->part, bt.S, i);
-        const FrameParams& fp = bt.fp[sc];
-        const int local = i - bt.off->part[sc];
-        keys[i] = ((uint32_t)sc << 24) | one_minus_u01_key(resample_word(fp.seed, fp.frame, (uint64_t)local));
-    }
-}
-
-int draw_key_bits(int S) {
-    int b = 0;
-    while ((1 << b) < S) ++b;
-    return 24 + b;
-}
-
-void launch_draw_keys(const Batch& bt, uint32_t* keys, cudaStream_t st) {
-    if (bt.P <= 0) return;
-    ++g_launches;
-    k_draw_keys<<<grid_for(bt.P), kBlock, 0, st>>>(bt, keys);
-}
-
 constexpr int kResThreads = 256;
 
 // calc_resampled_indices + resamplingKernel (resampling.cu:55-89): ancestor =
@@ -567,7 +541,7 @@ struct ResScene {
         return lo;
     }
     __device__ __forceinline__ float draw(int k) const {  // k local
-        const float om = (float)(dk[k] & 0xFFFFFFu) * 5.9604644775390625e-08f;
+        const float om = (float)dk[k] * 5.9604644775390625e-08f;
         return __fadd_rn(0.0f, __fmul_rn(jmax, om));
     }
 };
@@ -580,7 +554,7 @@ __device__ __forceinline__ ResScene res_scene(const Batch& bt, const float* join
     r.cum = joint_cum + bt.off->joint[sc];
     r.dk = dkeys + bt.off->part[sc];
     r.jmax = r.cum[r.n - 1];
-    const float om_max = (float)(r.dk[r.P - 1] & 0xFFFFFFu) * 5.9604644775390625e-08f;
+    const float om_max = (float)r.dk[r.P - 1] * 5.9604644775390625e-08f;
     r.rmax = __fadd_rn(0.0f, __fmul_rn(r.jmax, om_max));
     return r;
 }
