@@ -101,7 +101,7 @@ struct k3dom_handle {
 
     cudaStream_t st = nullptr, st2 = nullptr, st3 = nullptr;  // frame; resampling draws; ray lists
     cudaStream_t st4 = nullptr;                               // registered output export
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_bin = nullptr, ev_cells = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_bin = nullptr, ev_cells = nullptr, ev_clear = nullptr;
     cudaEvent_t ev_out = nullptr, ev_out_done = nullptr;
     // registered output (k3dom_set_output): one cell field of one scene, written every frame
     int out_field = -1, out_scene = 0;
@@ -238,6 +238,7 @@ struct k3dom_handle {
         if (ev_join) cudaEventDestroy(ev_join);
         if (ev_bin) cudaEventDestroy(ev_bin);
         if (ev_cells) cudaEventDestroy(ev_cells);
+        if (ev_clear) cudaEventDestroy(ev_clear);
         if (ev_staged) cudaEventDestroy(ev_staged);
         if (ev_out) cudaEventDestroy(ev_out);
         if (ev_out_done) cudaEventDestroy(ev_out_done);
@@ -687,19 +688,28 @@ cudaError_t enq_predict(k3dom_handle* h) {
     return cudaGetLastError();
 }
 
-cudaError_t enq_assign(k3dom_handle* h) {
+// The sort's scratch and the cell ranges to their start values (before an assignment): a frame does
+// this on its second stream, beside prediction.
+cudaError_t enq_clear_assign(k3dom_handle* h, cudaStream_t s) {
+    cudaError_t e = onesweep_clear(h->os_scratch, h->P, key_bits_for(h->C), s);
+    if (e != cudaSuccess) return e;
+    return cudaMemsetAsync(h->cw.start, 0xFF, 2 * sizeof(int) * (size_t)h->C, s);  // start and end
+}
+
+cudaError_t enq_assign(k3dom_handle* h, bool cleared = false) {
     // the records the gather reads (prediction wrote them; otherwise packed from A, whose cell
     // indices are always current)
     if (!h->x_current) {
         launch_pack_records(h->P, h->A, h->X, h->st);
         h->x_current = true;
     }
-    cudaError_t e = onesweep_sort_pairs(reinterpret_cast<const uint32_t*>(h->A.cell), nullptr, h->sorted_keys,
-                                        h->perm, h->alt_k, h->alt_v, h->P, key_bits_for(h->C), h->os_scratch,
-                                        h->os_words, h->status, h->sort_wait, h->st);
+    cudaError_t e = cleared ? cudaSuccess : enq_clear_assign(h, h->st);
     if (e != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(h->cw.start, 0xFF, sizeof(int) * (size_t)h->C, h->st))) return e;
-    if ((e = cudaMemsetAsync(h->cw.end, 0xFF, sizeof(int) * (size_t)h->C, h->st))) return e;
+    SortWait w = h->sort_wait;
+    w.cleared = true;
+    e = onesweep_sort_pairs(reinterpret_cast<const uint32_t*>(h->A.cell), nullptr, h->sorted_keys, h->perm, h->alt_k,
+                            h->alt_v, h->P, key_bits_for(h->C), h->os_scratch, h->os_words, h->status, w, h->st);
+    if (e != cudaSuccess) return e;
     launch_gather_segsum(h->batch(), h->X, h->Ss, h->sorted_keys, h->perm, h->cw, h->seg_rec, h->st);
     return cudaGetLastError();
 }
@@ -800,6 +810,8 @@ cudaError_t enq_frame(k3dom_handle* h) {
     const long l0 = g_launches;
     // resampling draws depend only on (seed, frame): produce them beside the frame
     if ((e = cudaEventRecord(h->ev_fork, h->st))) return e;
+    if ((e = cudaStreamWaitEvent(h->st4, h->ev_fork, 0))) return e;
+    if ((e = enq_clear_assign(h, h->st4)) || (e = cudaEventRecord(h->ev_clear, h->st4))) return e;
     if ((e = cudaStreamWaitEvent(h->st2, h->ev_fork, 0))) return e;
     if ((e = enq_draws(h, h->st2))) return e;
     if ((e = cudaEventRecord(h->ev_join, h->st2))) return e;
@@ -818,7 +830,7 @@ cudaError_t enq_frame(k3dom_handle* h) {
     rec(h, 0);
     if ((e = enq_predict(h))) return e;
     rec(h, 1);
-    if ((e = enq_assign(h))) return e;
+    if ((e = cudaStreamWaitEvent(h->st, h->ev_clear, 0)) || (e = enq_assign(h, true))) return e;
     rec(h, 2);
     if (overlap) {
         if ((e = cudaStreamWaitEvent(h->st, h->ev_bin, 0))) return e;
@@ -1001,6 +1013,7 @@ k3dom_status k3dom_batch_create(const k3dom_params* params, int32_t n_scenes, k3
     std::memset(h->status_host, 0, sizeof(DevStatus));
     if ((e = cudaEventCreateWithFlags(&h->ev_bin, cudaEventDisableTiming))) return bail(e);
     if ((e = cudaEventCreateWithFlags(&h->ev_cells, cudaEventDisableTiming))) return bail(e);
+    if ((e = cudaEventCreateWithFlags(&h->ev_clear, cudaEventDisableTiming))) return bail(e);
     if ((e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming))) return bail(e);
     if ((e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming))) return bail(e);
     if ((e = cudaEventCreateWithFlags(&h->ev_staged, cudaEventDisableTiming))) return bail(e);
@@ -1022,7 +1035,9 @@ k3dom_status k3dom_batch_create(const k3dom_params* params, int32_t n_scenes, k3
         return bail(e);
     if ((e = h->alloc_cells(&h->cs[0], C)) || (e = h->alloc_cells(&h->cs[1], C))) return bail(e);
     CellWork& cw = h->cw;
-    if ((e = h->alloc(&cw.start, C)) || (e = h->alloc(&cw.end, C)) || (e = h->alloc(&h->start2, C)) ||
+    if ((e = h->alloc(&cw.start, 2 * (size_t)C))) return bail(e);
+    cw.end = cw.start + C;  // one array, cleared together
+    if ((e = h->alloc(&h->start2, C)) ||
         (e = h->alloc(&h->end2, C)) || (e = h->alloc(&cw.sum_w, C)) || (e = h->alloc(&cw.sum_wvx, C)) ||
         (e = h->alloc(&cw.sum_wvy, C)) || (e = h->alloc(&cw.sum_wvz, C)) || (e = h->alloc(&cw.factor, C)) ||
         (e = h->alloc(&cw.divisor, C)) || (e = h->alloc(&cw.meas_occ, C)) || (e = h->alloc(&cw.meas_free, C)) ||

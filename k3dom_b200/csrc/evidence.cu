@@ -2366,8 +2366,12 @@ __global__ void __launch_bounds__(kBlock) k_k3dom_update_cells(EvArgs A) {
 // launcher) and a full tile starts at a multiple of 4 KB, as the copies require; the last, partial
 // tile reads its cells directly. The wait is bounded: when it runs out the CTA records
 // copy_timeout, waits (bounded again) for its copies to land, and skips its cells.
+// Maps below kUcBulk cells take the plain kernel: a CTA per 1,024 cells leaves too few of them to
+// hide the copies' latency (8k cells 10.1 -> 4.0 us, 120k 11.3 -> 6.1, 1.2M 30.0 -> 23.7, 1M equal;
+// 2.1M cells are 65 us that way and 56 by copies).
 constexpr int kUcCells = 1024;
 constexpr int kUcThreads = 256;
+constexpr int kUcBulk = 1500000;
 constexpr uint32_t kUcMaxPolls = 1u << 22;
 constexpr size_t kUcSmem = 8 * sizeof(float) * kUcCells + sizeof(ulonglong2) * kUcCells;
 
@@ -2493,7 +2497,7 @@ cudaError_t launch_k3dom_update_cells(const Batch& bt, RayBuffers& rb, CellState
                             reinterpret_cast<uintptr_t>(cw.sum_w) | reinterpret_cast<uintptr_t>(cw.sum_wvx) |
                             reinterpret_cast<uintptr_t>(cw.sum_wvy) | reinterpret_cast<uintptr_t>(cw.sum_wvz) |
                             reinterpret_cast<uintptr_t>(rb.acc);
-    if ((bases & 15u) == 0) {  // the bulk copies' alignment (cudaMalloc gives 256 bytes)
+    if (bt.C >= kUcBulk && (bases & 15u) == 0) {  // the bulk copies' alignment (cudaMalloc gives 256 bytes)
         k_k3dom_update_cells_bulk<<<div_up(bt.C, kUcCells), kUcThreads, kUcSmem, st>>>(A);
         return cudaGetLastError();
     }

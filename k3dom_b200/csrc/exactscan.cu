@@ -141,18 +141,29 @@ __device__ __forceinline__ u128 group_prefix(const u128* __restrict__ gsum, int 
     return r;
 }
 
+// Plans of up to kExDirect tiles skip the group pass: each apply CTA adds up its segment's earlier tile
+// sums itself (8 KB on average from L2 at the limit), which is one launch less on the frame's critical
+// path (4 us at 8k..2M cells; at the limit the two ways cost the same 20 us).
+constexpr int kExDirect = 1024;
+
 // 4 CTAs per SM (64 registers): the pass waits on its loads with few warps otherwise. CLEAR: the
 // tile's sign-bit inputs (which the scan counts as 0) are set to +0 in place.
-template <bool CLEAR>
+template <bool CLEAR, bool DIRECT>
 __global__ void __launch_bounds__(kExThreads, 4) exact_tab_apply(const ExactTile* __restrict__ tiles, int nt,
                                                                 const u128* __restrict__ tsum,
                                 const u128* __restrict__ gsum) {
     __shared__ u128 sm[kExThreads / 32 + 1];
     const int b = blockIdx.x;
     const ExactTile t = tiles[b];
-    const u128 pre_b = group_prefix(gsum, b / kExGroup) + tsum[b];
     const int f = t.seg_first;
-    const u128 pre_f = group_prefix(gsum, f / kExGroup) + tsum[f];
+    u128 before;  // the segment's sum before this tile
+    if (DIRECT) {
+        u128 s = 0;
+        for (int i = f + (int)threadIdx.x; i < b; i += kExThreads) s += tsum[i];
+        block_exclusive_scan<u128, kExThreads>(s, sm, &before);
+    } else {
+        before = group_prefix(gsum, b / kExGroup) + tsum[b] - (group_prefix(gsum, f / kExGroup) + tsum[f]);
+    }
     const int base = threadIdx.x * kExItems;
     // the inputs stay in registers as floats and are converted twice (cheaper than holding
     // eight 128-bit values across the block scan)
@@ -178,7 +189,7 @@ __global__ void __launch_bounds__(kExThreads, 4) exact_tab_apply(const ExactTile
 #pragma unroll
     for (int j = 0; j < kExItems; ++j) s += to_fixed(x[j]);
     u128 tot;
-    u128 run = (pre_b - pre_f) + block_exclusive_scan<u128, kExThreads>(s, sm, &tot);
+    u128 run = before + block_exclusive_scan<u128, kExThreads>(s, sm, &tot);
     float y[kExItems];
 #pragma unroll
     for (int j = 0; j < kExItems; ++j) {
@@ -222,16 +233,17 @@ cudaError_t exact_scan_plan(const ExactTile* tiles, int nt, void* scratch, cudaS
     if (nt <= 0) return cudaSuccess;
     u128* tsum = reinterpret_cast<u128*>(scratch);
     u128* gsum = tsum + nt;
-    const int ng = div_up(nt, kExGroup);
+    const bool direct = nt <= kExDirect;
     ++g_launches;
     exact_tab_sums<<<nt, kExThreads, 0, st>>>(tiles, nt, tsum);
+    if (!direct) {
+        ++g_launches;
+        exact_tab_groups<<<div_up(nt, kExGroup), kExThreads, 0, st>>>(tsum, nt, gsum);
+    }
     ++g_launches;
-    exact_tab_groups<<<ng, kExThreads, 0, st>>>(tsum, nt, gsum);
-    ++g_launches;
-    if (clear_signed)
-        exact_tab_apply<true><<<nt, kExThreads, 0, st>>>(tiles, nt, tsum, gsum);
-    else
-        exact_tab_apply<false><<<nt, kExThreads, 0, st>>>(tiles, nt, tsum, gsum);
+    auto apply = clear_signed ? (direct ? exact_tab_apply<true, true> : exact_tab_apply<true, false>)
+                              : (direct ? exact_tab_apply<false, true> : exact_tab_apply<false, false>);
+    apply<<<nt, kExThreads, 0, st>>>(tiles, nt, tsum, gsum);
     return cudaGetLastError();
 }
 

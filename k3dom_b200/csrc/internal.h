@@ -42,9 +42,11 @@ cudaError_t sort_init();
 struct SortWait {
     uint32_t max_polls = 1u << 20;
     int skip_tile = -1;
+    bool cleared = false;  // the caller has cleared the scratch (onesweep_clear)
 };
 int onesweep_plan(int key_bits, int* pass_bits);
 long onesweep_scratch_words(long n, int key_bits);
+cudaError_t onesweep_clear(uint32_t* scratch, long n, int key_bits, cudaStream_t st);
 cudaError_t onesweep_init();
 cudaError_t onesweep_sort_pairs(const uint32_t* keys, const uint32_t* vals, uint32_t* keys_out, uint32_t* vals_out,
                                 uint32_t* alt_k, uint32_t* alt_v, long n, int key_bits, uint32_t* scratch,

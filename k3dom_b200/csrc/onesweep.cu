@@ -18,14 +18,12 @@
 //    look-back, so later tiles count past it), so the output holds the keys and values of the
 //    completed tiles and in-range old contents elsewhere; the later passes then write nothing.
 // Digits of up to 8 bits, a key of b bits taking ceil(b / 8) passes of (nearly) equal width:
-// the 21-bit cell keys of 2^21 voxels three passes of 7 bits, the 24-bit resampling draws three
-// of 8 (four passes of 6 before: the draws' sort runs beside the particle sort and slowed it);
+// the 21-bit cell keys of 2^21 voxels three passes of 7 bits;
 // up to 256 digits per tile keep the runs long enough for coalesced writes. The element count
 // may live in device memory (`dn`, capped at nmax): the grid and scratch are sized for nmax,
 // CTAs whose tile lies past the live count return, and since tiles are handed out in order no
 // CTA waits on one of them. The same
-// sort orders the resampling draws (keys only) and the ray lists (tile of each entry, stable so
-// each tile keeps its rays in input order).
+// sort orders the ray lists (tile of each entry, stable so each tile keeps its rays in input order).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -80,6 +78,12 @@ long onesweep_scratch_words(long n, int key_bits) {
     const int np = onesweep_plan(key_bits, pb);
     const long tiles = div_up(std::max(n, 1L), (long)kOsTile);
     return (kOsMaxPasses + 1) + 2L * np * kOsDigits + (long)np * tiles * kOsDigits;
+}
+
+// The scratch's start state; a caller that clears ahead of time (beside other work) says so in its
+// SortWait.
+cudaError_t onesweep_clear(uint32_t* scratch, long n, int key_bits, cudaStream_t st) {
+    return cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * (size_t)onesweep_scratch_words(n, key_bits), st);
 }
 
 // A tile's status word carries its flag and its count together and guards no other data, so
@@ -368,8 +372,8 @@ cudaError_t onesweep_sort_pairs_dn(const uint32_t* keys, const uint32_t* vals, u
         shift += ps.bits[p];
     }
     const OsScratch sc = os_layout(scratch, ps.np);
-    cudaError_t e = cudaMemsetAsync(scratch, 0, sizeof(uint32_t) * (size_t)onesweep_scratch_words(n, key_bits), st);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = cudaSuccess;
+    if (!wait.cleared && (e = onesweep_clear(scratch, n, key_bits, st))) return e;
     ++g_launches;
     const long hist_grid = std::min((long)kOsHistBlocks, (long)div_up(n, (long)kOsThreads));
     os_hist<<<(unsigned)hist_grid, kOsThreads, 0, st>>>(keys, n, dn, ps, sc);

@@ -559,10 +559,14 @@ __device__ __forceinline__ ResScene res_scene(const Batch& bt, const float* join
     return r;
 }
 
+// Draws per thread: four keep more gathers in flight, but make too few blocks for the GPU below
+// kResWide particles, where one draw per thread is taken (16k particles 10.3 -> 4.5 us, 262k 14.8 -> 7.6,
+// 1M 25.4 -> 21.9; 2.5M are faster with four).
 constexpr int kResPerThread = 4;
-constexpr int kResBlock = kResThreads * kResPerThread;  // draws per resampling block
+constexpr int kResWide = 2000000;
+static int res_block(int P) { return kResThreads * (P < kResWide ? 1 : kResPerThread); }
 
-long res_bracket_count(long P) { return P > 0 ? div_up(P, (long)kResBlock) : 1; }
+long res_bracket_count(long P) { return P > 0 ? div_up(P, (long)kResThreads) : 1; }
 
 // The block's draws are sorted, so its ancestors lie in [lower(first draw), lower(last draw)]:
 // one warp per end of each block's bracket (all blocks in parallel). joint_cum is an exactly
@@ -572,13 +576,13 @@ long res_bracket_count(long P) { return P > 0 ? div_up(P, (long)kResBlock) : 1; 
 // returns the same index as the binary search. A block whose draws span two scenes gets
 // (-1, -1) and searches each draw in full.
 __global__ void k_res_brackets(Batch bt, const float* __restrict__ joint_cum, const uint32_t* __restrict__ dkeys,
-                               int nblocks, int* __restrict__ br) {
+                               int nblocks, int block, int* __restrict__ br) {
     const int w = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     const int blk = w >> 1, end = w & 1;
     if (blk >= nblocks) return;  // whole warps leave together
-    const int k0 = blk * kResBlock;
-    const int k1 = min(k0 + kResBlock, bt.P) - 1;
+    const int k0 = blk * block;
+    const int k1 = min(k0 + block, bt.P) - 1;
     const int sc = scene_of(bt.off->part, bt.S, k0);
     if (scene_of(bt.off->part, bt.S, k1) != sc) {
         if (lane == 0) br[w] = -1;
@@ -639,11 +643,12 @@ __device__ __forceinline__ void res_store(const ResScene& r, int k, int a, const
 
 // 5 CTAs per SM (48 registers, no spills): the gathers through the ancestor index wait on memory
 // latency, so more resident warps help.
+template <int PER>
 __global__ void __launch_bounds__(kResThreads, 5)
 k_resample(Batch bt, const float* __restrict__ joint_cum, const uint32_t* __restrict__ dkeys, const int2* br,
            Particles s, Particles b, Particles out, int* __restrict__ anc_out, float* __restrict__ joint_max_out) {
     __shared__ float s_acc[kResStage];
-    const int k0 = blockIdx.x * kResBlock;
+    const int k0 = blockIdx.x * (kResThreads * PER);
     const int2 bk = br[blockIdx.x];
     if (bk.x >= 0) {
         const int sc = scene_of(bt.off->part, bt.S, k0);
@@ -656,9 +661,9 @@ k_resample(Batch bt, const float* __restrict__ joint_cum, const uint32_t* __rest
             for (int i = threadIdx.x; i < len; i += kResThreads) s_acc[i] = r.acc(lo + i);
             __syncthreads();
         }
-        int a[kResPerThread];
+        int a[PER];
 #pragma unroll
-        for (int it = 0; it < kResPerThread; ++it) {
+        for (int it = 0; it < PER; ++it) {
             const int k = k0 + it * kResThreads + threadIdx.x;
             a[it] = 0;
             if (k >= bt.P) continue;
@@ -674,19 +679,19 @@ k_resample(Batch bt, const float* __restrict__ joint_cum, const uint32_t* __rest
                 a[it] = res_clamp(r, r.lower(u, lo, hi));
             }
         }
-        ResPart v[kResPerThread];
+        ResPart v[PER];
 #pragma unroll
-        for (int it = 0; it < kResPerThread; ++it)
+        for (int it = 0; it < PER; ++it)
             if (k0 + it * kResThreads + (int)threadIdx.x < bt.P) v[it] = res_load(bt, r, sc, a[it], s, b);
 #pragma unroll
-        for (int it = 0; it < kResPerThread; ++it) {
+        for (int it = 0; it < PER; ++it) {
             const int k = k0 + it * kResThreads + threadIdx.x;
             if (k >= bt.P) continue;
             res_store(r, k, a[it], v[it], out, anc_out);
             if (k == base && joint_max_out) joint_max_out[sc] = r.jmax;
         }
     } else {
-        for (int it = 0; it < kResPerThread; ++it) {
+        for (int it = 0; it < PER; ++it) {
             const int k = k0 + it * kResThreads + threadIdx.x;
             if (k >= bt.P) break;
             const int sc = scene_of(bt.off->part, bt.S, k);
@@ -703,12 +708,12 @@ void launch_resample(const Batch& bt, const float* joint_cum, const uint32_t* so
                      Particles b, Particles out, int* ancestors, float* joint_max_out, int2* brackets,
                      cudaStream_t st) {
     if (bt.P <= 0) return;
-    const int nblk = div_up(bt.P, kResBlock);
+    const int block = res_block(bt.P), nblk = div_up(bt.P, block);
     g_launches += 2;
-    k_res_brackets<<<div_up(nblk * 64, 256), 256, 0, st>>>(bt, joint_cum, sorted_draws, nblk,
+    k_res_brackets<<<div_up(nblk * 64, 256), 256, 0, st>>>(bt, joint_cum, sorted_draws, nblk, block,
                                                            reinterpret_cast<int*>(brackets));
-    k_resample<<<nblk, kResThreads, 0, st>>>(bt, joint_cum, sorted_draws, brackets, s, b, out, ancestors,
-                                             joint_max_out);
+    auto kern = block == kResThreads ? k_resample<1> : k_resample<kResPerThread>;
+    kern<<<nblk, kResThreads, 0, st>>>(bt, joint_cum, sorted_draws, brackets, s, b, out, ancestors, joint_max_out);
 }
 
 // ---------------------------------------------------------------- debug draws
