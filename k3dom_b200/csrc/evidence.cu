@@ -1192,13 +1192,16 @@ __device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
 // value and a batch per 32 listed rays 1.51 ms; the units' sums by additions, the interior class and
 // full batches 1.38 ms; two cells per lane 1.24 ms; four 1.20 ms (200x200x25 voxels at 0.2 m, 60,000
 // rays, ls 0.5 m: 0.54 -> 0.42 ms). The warp instructions per evaluation went from 4.2 to 3.2; what
-// is left is the table's gathers (half of the L1 data path) and the waits on them. Slower here: the
+// is left is the table's gathers (half of the L1 data path) and the waits on them. Two registers
+// fewer for the tests (two limits and NaN columns instead of four limits) end the spills: evidence
+// 1.19 -> 1.14 ms, the frame 1.745 -> 1.672. Slower here: the
 // table in shared memory (1.38 ms), predicated fetches for all cells at once (spills at 64 registers,
 // and 1.36 ms at 128 registers with 2 CTAs per SM), 3 CTAs per SM at 80 registers (1.21 ms).
 struct Cols {
     F2 EX, EY[2], EZ;  // anchor minus the cell centres: x, both y, z of the lower cells
     F2 TS;             // table scale
-    float ls2[4];      // ls^2 of cell (y, z) = (i & 1, i >> 1), -1 outside the grid
+    float ls2[2];      // ls^2 of the lower and the upper cells; -1 outside the grid (a column
+                       // outside it has NaN offsets, so no test on it is true)
 };
 
 // Squared perpendicular distances of the four cells to the lines of the two rays of a pair record
@@ -1337,7 +1340,7 @@ __device__ __forceinline__ void interior_batch(const EvArgs& A, const BgkiSmem& 
         for (int i = 0; i < 4; ++i) {
             float da, db;
             p.d2[i].split(da, db);
-            ev.free(i, tab_pos2(p.d2[i], C.TS), da < C.ls2[i], db < C.ls2[i]);
+            ev.free(i, tab_pos2(p.d2[i], C.TS), da < C.ls2[i >> 1], db < C.ls2[i >> 1]);
         }
     }
     ev.n_free += steps;
@@ -1386,7 +1389,7 @@ __device__ __forceinline__ void general_batch(const EvArgs& A, const BgkiSmem& S
                 const F2 w = i < 2 ? vl : vz;
                 const F2 d2 = fma2(w, w, fma2(vy, vy, xx));
                 d2.split(da, db);
-                ev.occ(i, tab_pos2(d2, C.TS), da < C.ls2[i], db < C.ls2[i]);
+                ev.occ(i, tab_pos2(d2, C.TS), da < C.ls2[i >> 1], db < C.ls2[i >> 1]);
             }
         }
         const Perp p = perp_d2(R, C);
@@ -1397,7 +1400,7 @@ __device__ __forceinline__ void general_batch(const EvArgs& A, const BgkiSmem& S
             float ea, eb;
             d2.split(da, db);
             sub2(F2::of(b5.z, b5.w), p.nd[i]).split(ea, eb);  // d_proj - d_m
-            ev.free(i, tab_pos2(d2, C.TS), ea < 0.0f && da < C.ls2[i], eb < 0.0f && db < C.ls2[i]);
+            ev.free(i, tab_pos2(d2, C.TS), ea < 0.0f && da < C.ls2[i >> 1], eb < 0.0f && db < C.ls2[i >> 1]);
         }
     }
     if (near_steps) ev.end_occ(near_steps);
@@ -1412,7 +1415,7 @@ __device__ __forceinline__ void general_batch(const EvArgs& A, const BgkiSmem& S
             const F2 d2 = along_d2(p.d2[i], b3, p.nd[i]);
             float da, db;
             d2.split(da, db);
-            ev.free(i, tab_pos2(d2, C.TS), da < C.ls2[i], db < C.ls2[i]);
+            ev.free(i, tab_pos2(d2, C.TS), da < C.ls2[i >> 1], db < C.ls2[i >> 1]);
         }
     }
     ev.n_free += steps;
@@ -1446,12 +1449,13 @@ __device__ __forceinline__ void eval_sub_block(const EvArgs& A, const BgkiSmem& 
         centre_xyz(ix, iy + 1, b.z, p, I.sx, I.sy, I.sz, &t, &y1, &t);
         centre_xyz(b.x + 2, b.y + 2, b.z + 1, p, I.sx, I.sy, I.sz, &ox, &oy, &oz);
         // exact (nearby floats)
-        const float ex = ox - x, ey0 = oy - y0, ey1 = oy - y1, ez = oz - z, ts = I.tscale;
+        const float nan = __int_as_float(0x7fffffff);
+        const float ex = ix < I.G ? ox - x : nan, ey0 = iy < I.G ? oy - y0 : nan, ey1 = iy + 1 < I.G ? oy - y1 : nan;
+        const float ez = oz - z, ts = I.tscale;
         C.EX = F2::of(ex, ex); C.EY[0] = F2::of(ey0, ey0); C.EY[1] = F2::of(ey1, ey1); C.EZ = F2::of(ez, ez);
         C.TS = F2::of(ts, ts);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            C.ls2[i] = ix < I.G && iy + (i & 1) < I.G && b.z + (i >> 1) < I.Gz ? I.ls2 : -1.0f;
+        C.ls2[0] = b.z < I.Gz ? I.ls2 : -1.0f;
+        C.ls2[1] = b.z + 1 < I.Gz ? I.ls2 : -1.0f;
     }
     ev.begin(I);
     uint16_t* gring = ring + kRing;
