@@ -532,7 +532,7 @@ cudaError_t alloc_ray_lane(k3dom_calib* c, RayBuffers& rb, int max_points, long 
         (e = c->alloc(&rb.evals2, cap, L)) || (e = c->alloc(&rb.tile_start, T + 1, L)) ||
         (e = c->alloc(&rb.item_off, T + 1, L)) || (e = c->alloc(&rb.tile_done, T, L)) || (e = c->alloc(&rb.total, 4, L)))
         return e;
-    if (placed_lists(false, T))  // lists placed per tile through tallies and per-block offsets
+    if (placed_lists(false, T, N))  // lists placed per tile through tallies and per-block offsets
         return (e = c->alloc(&rb.tile_tally, T, L))
                    ? e
                    : c->alloc(&rb.block_base, (size_t)bin_blocks((long)kRayThreads * N) * T, L);

@@ -403,9 +403,19 @@ cudaError_t alloc_ray_buffers(k3dom_handle* h) {
         (e = h->alloc(&rb.tile_done, T, true, L)) || (e = h->alloc(&rb.acc, 2 * (size_t)h->C, true, L)) ||
         (e = h->alloc(&rb.total, 4, true, L)))
         return e;
-    if (placed_lists(h->ds(), T)) {  // per-tile tallies and per-block offsets
-        if ((e = h->alloc(&rb.tile_tally, T, true, L)) ||
-            (e = h->alloc(&rb.block_base, (size_t)bin_blocks((long)kRayThreads * N) * T, true, L)))
+    if (h->ds()) {
+        h->ds_sized_chunk = std::max(32, h->chunk);
+        const long items_max = T + cap / h->ds_sized_chunk + 2;
+        rb.ds_stride = 1;
+        for (const SceneHost& x : h->sc) rb.ds_stride = std::max(rb.ds_stride, x.ts.tx * x.ts.ty * x.ts.tz);
+        rb.ds_capacity = items_max * rb.ds_stride;
+        if ((e = h->alloc(&rb.ds_counts, rb.ds_capacity, false, L)) || (e = h->alloc(&rb.ds_r2, rb.ds_capacity, false, L)))
+            return e;
+    }
+    if (placed_lists(h->ds(), T, N)) {  // per-tile tallies and per-block offsets or counts
+        const long blocks = h->ds() ? mark_blocks(N) : bin_blocks((long)kRayThreads * N);
+        if ((e = h->alloc(&rb.tile_tally, T, true, L)) || (e = h->alloc(&rb.block_base, (size_t)blocks * T, true, L)) ||
+            (h->ds() && (e = h->alloc(&rb.mark_groups, (size_t)mark_groups(N) * T, true, L))))
             return e;
         return alloc_points(h);
     }
@@ -423,15 +433,6 @@ cudaError_t alloc_ray_buffers(k3dom_handle* h) {
     } else {
         rb.ekeys_alt = rb.ekeys;
         rb.evals_alt = rb.evals;
-    }
-    if (h->ds()) {
-        h->ds_sized_chunk = std::max(32, h->chunk);
-        const long items_max = T + cap / h->ds_sized_chunk + 2;
-        rb.ds_stride = 1;
-        for (const SceneHost& x : h->sc) rb.ds_stride = std::max(rb.ds_stride, x.ts.tx * x.ts.ty * x.ts.tz);
-        rb.ds_capacity = items_max * rb.ds_stride;
-        if ((e = h->alloc(&rb.ds_counts, rb.ds_capacity, false, L)) || (e = h->alloc(&rb.ds_r2, rb.ds_capacity, false, L)))
-            return e;
     }
     rb.os_words = onesweep_scratch_words(cap, bits);
     rb.scan_words = scan_u32_tiles(std::max((long)N, (long)T + 1)) + 16;

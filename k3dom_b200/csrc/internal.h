@@ -143,14 +143,16 @@ struct RayBuffers {
     float4* ktab;          // per scene: sparse-kernel table with the fixed-point scale folded in
     cudaTextureObject_t ktex;  // the kernel table through the texture path (k_bgki: ktab; k_bgki_sums: f), 0 when not made
     uint32_t* counts;      // [kRayThreads * N] tiles touched per point slot (DS) or per thread of a slot
-    uint32_t* offsets;     // exclusive scan of counts (DS)
-    uint32_t* ekeys;       // entries: global tile id (DS)
-    uint32_t* evals;       // entries: point slot (DS)
-    uint32_t* ekeys2;      // sorted (DS)
-    uint32_t* evals2;      // the lists: point slots grouped by tile (K3DOM: placed, DS: sorted)
-    uint32_t* tile_tally;  // T: rays per tile (K3DOM), zero between frames
-    uint32_t* block_base;  // [bin_blocks(kRayThreads N)][T]: each binning block's first slot in each tile's range,
-                           // relative to the range's start (K3DOM)
+    uint32_t* offsets;     // exclusive scan of counts (sorted lists)
+    uint32_t* ekeys;       // entries: global tile id (sorted lists)
+    uint32_t* evals;       // entries: point slot (sorted lists)
+    uint32_t* ekeys2;      // sorted lists
+    uint32_t* evals2;      // the lists: point slots grouped by tile (placed or sorted)
+    uint32_t* tile_tally;  // T: rays per tile, zero between K3DOM frames
+    uint32_t* mark_groups;  // DS: [mark_groups(N)][T], counts per group of blocks, then their prefixes
+    uint32_t* block_base;  // DS: [mark_blocks(N)][T], rays per block and tile; K3DOM:
+                           // [bin_blocks(kRayThreads N)][T], each binning block's first slot in each
+                           // tile's range, relative to the range's start
     uint32_t* ekeys_alt;
     uint32_t* evals_alt;
     uint32_t* tile_start;  // T+1
@@ -172,10 +174,21 @@ struct RayBuffers {
     int item_slots;        // CTA slots the work items are spread over (0: items of chunk rays whatever the scene)
 };
 long ray_entries_bound(const DevParams& p, const TileShape& ts, int max_points, float bin_R);
-// K3DOM ray lists are placed per tile through block histograms of all T tiles in shared memory
-// (48 KB at most); DS lists, and batches with more tiles, are sorted by tile.
+// Ray lists are placed per tile through block histograms (K3DOM: 4 bytes a tile) or bit masks (DS: 16
+// bytes) of all T tiles in shared memory; otherwise the entries are sorted by tile. K3DOM takes up to
+// 48 KB, DS up to what lets two blocks share an SM (256x256x32 voxels, 120,000 rays: 1,024 tiles
+// placed 76 us, sorted 145; 2,048 tiles 94 and 156; 8,192 tiles, one block per SM, 271 and 229) and
+// up to kMarkMaxCounts counts (128 MB).
 constexpr int kPlacedMaxTiles = 12288;
-inline bool placed_lists(bool ds, int T) { return !ds && T <= kPlacedMaxTiles; }
+constexpr int kMarkMaxTiles = 6144;
+constexpr int kMarkRays = 128;   // rays per block of the DS passes
+constexpr int kMarkGroup = 32;   // blocks whose counts are added up together
+constexpr long kMarkMaxCounts = 32L << 20;
+int mark_blocks(int N);
+int mark_groups(int N);
+inline bool placed_lists(bool ds, int T, int N) {
+    return ds ? T <= kMarkMaxTiles && (long)mark_blocks(N) * T <= kMarkMaxCounts : T <= kPlacedMaxTiles;
+}
 constexpr int kBinBlocksMax = 1024;
 int bin_blocks(long n);  // blocks of the placed-list passes over n threads
 constexpr int kRayThreads = 2;  // threads per ray in the placed-list passes
