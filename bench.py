@@ -407,7 +407,7 @@ def evidence_roofline(m: dict, variant: str) -> dict:
     tr_file = ROOT / "profiles" / ("dsgrid_traffic.json" if ds else "bgki_traffic.json")
     rule_name = ["by-size", "8x8x4", "16x16x4", "16x16x8"][m["tuning"]["tile_rule"]]
     if rule_name == "by-size":
-        rule_name = "16x16x8"  # the rule's choice for grids of >= 2^20 cells
+        rule_name = "16x16x4"  # the rule's choice for K3DOM grids of >= 2^19 cells
     if tr_file.exists():
         try:
             d = json.loads(tr_file.read_text())
@@ -418,7 +418,7 @@ def evidence_roofline(m: dict, variant: str) -> dict:
         except Exception:
             traffic = None
     return {
-        "kernel": ("k_dsgrid (DS measurement grid + fused Dempster update)" if ds else
+        "kernel": ("k_ds_rays, k_ds_combine, k_ds_partial, k_ds_update (DS measurement grid and cell update)" if ds else
                    "k_bgki (sparse BGKI evidence + fused cell update)"),
         "bound": "fp32", "achieved": round(achieved, 3), "peak": round(NOMINAL_FP32_TFLOPS, 1),
         "unit": "TFLOP/s", "frac": round(achieved / NOMINAL_FP32_TFLOPS, 4), "traffic": traffic,

@@ -42,9 +42,20 @@ enum TileRule { kRuleBySize = 0, kRuleSmall = 1, kRuleFlat = 2, kRuleLarge = 3, 
 
 TileShape tile_shape(const DevParams& p, int rule) {
     int tx = 8, ty = 8, tz = 4;
-    const bool large = (long)p.C >= (1L << 20) && p.Gz >= 8;
+    // By size: larger tiles mean fewer list entries and fewer items, smaller ones more items for the
+    // GPU's slots. Frames in us with 8x8x4, 16x16x4, 16x16x8 tiles (0.1 to 0.2 m voxels, 60,000 and
+    // 120,000 rays): K3DOM 250k cells 447, 454, 480; 524k 652, 659, 718 and (0.2 m) 441, 433, 475; 1M
+    // 625, 621, 657; 1.05M 1138, 1083, 1168; 2.1M 1564, 1471, 1567; 3.2M 1118, 965, 1050. DS 250k 346,
+    // 327, 321; 524k 429, 412, 405; 1M 476, 434, 412; 2.1M 871, 766, 733.
+    const bool large = (long)p.C >= (p.variant != 0 ? 1L << 17 : 1L << 19);
     switch (rule) {
-        case kRuleBySize: if (large) { tx = 16; ty = 16; tz = 8; } break;
+        case kRuleBySize:
+            if (large) {
+                tx = 16;
+                ty = 16;
+                tz = p.variant != 0 && p.Gz >= 8 ? 8 : 4;
+            }
+            break;
         case kRuleSmall: break;
         case kRuleFlat: tx = 16; ty = 16; tz = 4; break;
         case kRuleLarge: tx = 16; ty = 16; tz = p.Gz >= 8 ? 8 : 4; break;
@@ -161,7 +172,7 @@ struct k3dom_handle {
 
     // evidence tuning
     int tile_rule = kRuleBySize;
-    int chunk = 1024;
+    int chunk = 1024;        // DS starts at 512 (200x200x25 voxels 412 -> 396 us, 2.1M cells equal)
     int tune_next = -1;  // next candidate to measure, -1 when not tuning
     float tune_best_ms = 0.0f;
     int tune_best = 0, tuned = 0;
@@ -959,6 +970,7 @@ k3dom_status k3dom_batch_create(const k3dom_params* params, int32_t n_scenes, k3
     if (!h) return K3DOM_ERR_OUT_OF_MEMORY;
     h->device = device;
     h->variant = variant;
+    if (h->ds()) h->chunk = 512;
     h->S = n_scenes;
     h->sc.resize(n_scenes);
     auto bail = [&](cudaError_t e) {
