@@ -2673,6 +2673,9 @@ cudaError_t evidence_init() {
     const int marks = (int)(sizeof(uint4) * kMarkMaxTiles);
     cudaError_t m = cudaFuncSetAttribute(k_ds_mark<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, marks);
     if (m == cudaSuccess) m = cudaFuncSetAttribute(k_ds_mark<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, marks);
+    const int hist = (int)(sizeof(uint32_t) * kPlacedMaxTiles);
+    if (m == cudaSuccess) m = cudaFuncSetAttribute(k_ray_count<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, hist);
+    if (m == cudaSuccess) m = cudaFuncSetAttribute(k_ray_place, cudaFuncAttributeMaxDynamicSharedMemorySize, hist);
     if (m != cudaSuccess) return m;
     cudaError_t e = cudaFuncSetAttribute(k_bgki, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)bgki_smem_bytes(kChunk));

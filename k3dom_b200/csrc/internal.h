@@ -175,11 +175,12 @@ struct RayBuffers {
 };
 long ray_entries_bound(const DevParams& p, const TileShape& ts, int max_points, float bin_R);
 // Ray lists are placed per tile through block histograms (K3DOM: 4 bytes a tile) or bit masks (DS: 16
-// bytes) of all T tiles in shared memory; otherwise the entries are sorted by tile. K3DOM takes up to
-// 48 KB, DS up to what lets two blocks share an SM (256x256x32 voxels, 120,000 rays: 1,024 tiles
-// placed 76 us, sorted 145; 2,048 tiles 94 and 156; 8,192 tiles, one block per SM, 271 and 229) and
-// up to kMarkMaxCounts counts (128 MB).
-constexpr int kPlacedMaxTiles = 12288;
+// bytes) of all T tiles in shared memory; otherwise the entries are sorted by tile. Both take what
+// lets two blocks share an SM. K3DOM batches of 4 to 11 uneven scenes, lists placed and sorted: 12,736
+// tiles 359 and 743 us, 17,429 574 and 1,112, 27,293 1,028 and 1,561, 36,449 (one block per SM) 2,212
+// and 2,108. DS, 256x256x32 voxels, 120,000 rays: 1,024 tiles 76 and 145 us, 2,048 94 and 156, 8,192
+// (one block) 271 and 229. DS keeps up to kMarkMaxCounts counts (128 MB).
+constexpr int kPlacedMaxTiles = 28416;
 constexpr int kMarkMaxTiles = 6144;
 constexpr int kMarkRays = 128;   // rays per block of the DS passes
 constexpr int kMarkGroup = 32;   // blocks whose counts are added up together
