@@ -41,7 +41,7 @@ struct SceneDev {
     int n_tiles, max_points;
     float bin_R;    // ray-binning support radius [cells] (DS: an upper bound, see ds_window)
     float wr2;       // DS window radius squared [m^2]
-    float cull_ls2;  // K3DOM: squared support radius of the sub-block cull, ls plus slack [m^2]
+    float cull_ls2;  // squared support radius of the sub-block cull [m^2]: ls plus slack (DS: bin_R)
     double fx_inv;   // K3DOM evidence: value = fixed-point integer * fx_inv
 };
 

@@ -55,6 +55,7 @@ constexpr int kFxShift = 40;  // fixed-point units of the K3DOM and calibration 
 struct BinGeom {
     float ax, ay, az;  // sensor in cell-index space (cell centre ix sits at u = ix)
     float R;           // support radius in cells
+    float R_far;       // DS: the radius for rays of ds_extreme
     int G, Gz, tx, ty, tz, ntx, nty, ntz;
 };
 
@@ -172,10 +173,18 @@ struct RayPrep {
     float bx, by, bz;  // far end of the binned segment (cell-index space)
 };
 
+// DS rays whose |m|^2 leaves [2^-80, 2^80] (points beyond 1e12 m, or within 1e-12 m of the sensor). The
+// reference's FP32 test overflows or underflows for them: with |m|^2 infinite it accepts the cells
+// around the sensor whatever the ray's direction, and with (c.m)^2 infinite cells beside the line. So
+// a window around the half-line does not hold their neighbours; they take every cell of the
+// sub-blocks near it (ds_reaches_sub_block), in lists of the widest radius.
+__device__ __forceinline__ bool ds_extreme(float sq) { return !(sq >= 8.2718061e-25f && sq <= 1.2089258e24f); }
+
 // Per-ray constants. K3DOM: (m, d_m) and (m/d_m, margin), d_m and margin as the reference
 // forms them (mass_update.cu:29-31,55). DS: (m, |m|^2) as measurement_grid.cu:90.
 // consts = false: only ok and the segment's far end (K3DOM), for a second thread of the ray.
-__device__ __forceinline__ RayPrep prep_ray(const DevParams& p, const BinGeom& g, float mx, float my, float mz,
+// A ray of ds_extreme widens g.R.
+__device__ __forceinline__ RayPrep prep_ray(const DevParams& p, BinGeom& g, float mx, float my, float mz,
                                            bool ds, float4* ra, double4* rc, bool consts = true) {
     RayPrep r;
     r.ok = isfinite(mx) && isfinite(my) && isfinite(mz);
@@ -207,6 +216,7 @@ __device__ __forceinline__ RayPrep prep_ray(const DevParams& p, const BinGeom& g
             r.ok = false;  // |m| = 0: inner product 0, never a neighbour (measurement_grid.cu:92)
             return r;
         }
+        if (ds_extreme(sq)) g.R = g.R_far;
         // length of the binned half-line in cells: past the grid's far corner, also from a sensor
         // outside the grid
         const float diag = sqrtf((float)(2 * g.G * g.G + g.Gz * g.Gz));
@@ -233,7 +243,7 @@ __device__ __forceinline__ float ds_window(float wr2, float dist2, float res) {
 
 __device__ __forceinline__ BinGeom scene_geom(const SceneDev& sd, const FrameParams& f) {
     BinGeom g;
-    g.R = sd.bin_R;
+    g.R = g.R_far = sd.bin_R;
     if (sd.p.variant != 0) {  // DS: from the farthest cell
         const float ext = sqrtf(f.sensor_x * f.sensor_x + f.sensor_y * f.sensor_y + f.sensor_z * f.sensor_z) +
                           0.5f * sd.p.res * sqrtf((float)(2 * sd.p.G * sd.p.G + sd.p.Gz * sd.p.Gz));
@@ -278,7 +288,7 @@ __global__ void k_ray_count(Batch bt, const float* __restrict__ xs, const float*
             continue;
         }
         const SceneDev& sd = bt.sc[sc];
-        const BinGeom g = scene_geom(sd, f);
+        BinGeom g = scene_geom(sd, f);
         float mx = xs[i], my = ys[i], mz = zs[i];
         if (f.has_transform) apply_transform(f, &mx, &my, &mz);
         float4 a;
@@ -329,7 +339,7 @@ __global__ void k_ray_emit(Batch bt, const float* __restrict__ xs, const float* 
         const FrameParams f = bt.fp[sc];
         if (i - bt.off->point[sc] >= f.n_points) continue;
         const SceneDev& sd = bt.sc[sc];
-        const BinGeom g = scene_geom(sd, f);
+        BinGeom g = scene_geom(sd, f);
         float mx = xs[i], my = ys[i], mz = zs[i];
         if (f.has_transform) apply_transform(f, &mx, &my, &mz);
         float4 a;
@@ -541,7 +551,7 @@ k_ds_mark(Batch bt, const float* __restrict__ xs, const float* __restrict__ ys, 
     if (i < bt.N && i - bt.off->point[sc] < bt.fp[sc].n_points) {
         const FrameParams f = bt.fp[sc];
         const SceneDev& sd = bt.sc[sc];
-        const BinGeom g = scene_geom(sd, f);
+        BinGeom g = scene_geom(sd, f);
         float mx = xs[i], my = ys[i], mz = zs[i];
         if (f.has_transform) apply_transform(f, &mx, &my, &mz);
         float4 a;
@@ -637,8 +647,8 @@ void fill_scene_evidence(SceneDev& sd, bool ds, float4* ktab) {
         sd.bin_R = sqrtf(p.window_radius * p.window_radius + slack) / p.res + 1e-3f;
     }
     sd.wr2 = p.window_radius * p.window_radius;
-    // K3DOM box culls (box_reaches): the support radius with a margin
-    const float rls = p.ls * (1.0f + 1e-4f) + 1e-3f * p.res;
+    // box culls (box_reaches): the support radius with a margin; DS (rays of ds_extreme): bin_R in metres
+    const float rls = ds ? sd.bin_R * p.res : p.ls * (1.0f + 1e-4f) + 1e-3f * p.res;
     sd.cull_ls2 = rls * rls;
     // fixed point: the table is scaled by a power of two so that a kernel value is at most 1, and
     // one unit is 2^-40 of that: at most 2^40 units a value, leaving 2^23 terms of headroom in a
@@ -2039,6 +2049,47 @@ __device__ __forceinline__ void ds_layer(DsTile& S, const TileShape& ts, const D
     }
 }
 
+// Whether a ray of ds_extreme takes the cells of the sub-block with centroid (qx, qy, qz): the box
+// bound (box_reaches) on the distance from its half-line, in the FP32 arithmetic whose direction is
+// zero for an infinite |m|^2 (then the half-line is the sensor). It does not depend on the tiling.
+__device__ __forceinline__ bool ds_reaches_sub_block(float qx, float qy, float qz, const float4& m, float hres,
+                                                     float rls2) {
+    const float len = sqrtf(m.w), inv = len > 0.0f ? 1.0f / len : 0.0f;
+    const float ux = m.x * inv, uy = m.y * inv, uz = m.z * inv;
+    const float t = fmaxf(qx * ux + qy * uy + qz * uz, 0.0f);
+    const float Dx = qx - t * ux, Dy = qy - t * uy, Dz = qz - t * uz;
+    return box_reaches(Dx, Dy, Dz, Dx * Dx + Dy * Dy + Dz * Dz, hres, rls2);
+}
+
+// A ray of ds_extreme in the tile, by a warp: the reference's test on every cell of the sub-blocks near
+// its half-line. Such rays are too rare to be worth more (a sensor's far-away marker for no return).
+__device__ __noinline__ void ds_extreme_ray(DsTile& S, const ItemConst& I, const float4& mr, float wr2) {
+    const TileShape& ts = I.ts;
+    const float4 m = mr;
+    const float hres = 0.5f * I.res, rls2 = I.rls2;
+    const int lane = threadIdx.x & 31;
+    for (int s0 = 0; s0 < I.nsb; s0 += 32) {
+        const int sb = s0 + lane;
+        bool hit = false;
+        if (sb < I.nsb) {
+            const SbCell b = sb_cell(ts, 0, sb);
+            hit = ds_reaches_sub_block(S.c[0][b.x + 2].x - hres, S.c[1][b.y + 2].x - hres, S.c[2][b.z + 1].x - hres, m,
+                                       hres, rls2);
+        }
+        for (unsigned left = __ballot_sync(0xffffffffu, hit); left; left &= left - 1u) {
+            const SbCell b = sb_cell(ts, 0, s0 + __ffs(left) - 1);
+            const int x = b.x + (lane & 3), y = b.y + ((lane >> 2) & 3), z = b.z + (lane >> 4);
+            if (x >= S.n[0] || y >= S.n[1] || z >= S.n[2]) continue;
+            const float2 cx = S.c[0][x], cy = S.c[1][y], cz = S.c[2][z];
+            const float acs = __fadd_rn(__fadd_rn(cx.y, cy.y), cz.y);
+            if (!ds_is_neighbor(cx.x, cy.x, cz.x, acs, m, wr2)) continue;
+            const int li = x + ts.tx * (y + ts.ty * z);
+            atomicAdd(&S.cf[li], acs > m.w ? 1u + kDsCloser : 1u);
+            atomicMin(&S.r2[li], __float_as_uint(ds_r_sqr(cx.x, cy.x, cz.x, m)));
+        }
+    }
+}
+
 __global__ void __launch_bounds__(kEvThreads) k_ds_rays(EvArgs A) {
     __shared__ ItemConst I;
     __shared__ DsTile S;
@@ -2088,11 +2139,14 @@ __global__ void __launch_bounds__(kEvThreads) k_ds_rays(EvArgs A) {
             for (int g = wid * 32; g < I.nr; g += kEvThreads) {
                 // one ray per lane: its line and layers; then one (ray, layer) per lane
                 int2 ly = make_int2(0, -1);
+                bool extreme = false;
                 if (g + lane < I.nr) {
                     uint32_t rid = A.evals[I.e0 + g + lane];
                     if (rid >= (uint32_t)bt.N) rid = 0;  // defensive: never read past the ray arrays
                     const float4 m = A.ray_a[rid];
-                    if (m.w > 0.0f) ly = ds_line(S, a, m, R, &W.ray[lane]);
+                    extreme = m.w > 0.0f && ds_extreme(m.w);
+                    if (extreme) W.ray[lane].m = m;
+                    else if (m.w > 0.0f) ly = ds_line(S, a, m, R, &W.ray[lane]);
                 }
                 const int n = max(ly.y - ly.x + 1, 0);
                 int end = n;  // inclusive prefix over the lanes
@@ -2111,6 +2165,8 @@ __global__ void __launch_bounds__(kEvThreads) k_ds_rays(EvArgs A) {
                     if (ax == 2) ds_layer<true>(S, ts, r, 2, e >> 5, wr2);
                     else ds_layer<false>(S, ts, r, ax, e >> 5, wr2);
                 }
+                for (unsigned left = __ballot_sync(0xffffffffu, extreme); left; left &= left - 1u)
+                    ds_extreme_ray(S, I, W.ray[__ffs(left) - 1].m, wr2);
                 __syncwarp();
             }
         }
@@ -2233,6 +2289,11 @@ __global__ void __launch_bounds__(kEvThreads) k_ds_partial(EvArgs A) {
         const float acs = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
         const uint32_t e0 = A.tile_start[t] + (item - first) * (uint32_t)A.chunk;
         const uint32_t e1 = min(A.tile_start[t + 1], e0 + (uint32_t)A.chunk);
+        const float hres = 0.5f * sd.p.res;
+        float qx, qy, qz;  // centroid of the cell's sub-block
+        centre_xyz((ix & ~3) + 2, (iy & ~3) + 2, (iz & ~1) + 1, sd.p, fp.sensor_x, fp.sensor_y, fp.sensor_z, &qx, &qy,
+                   &qz);
+        qx -= hres; qy -= hres; qz -= hres;
         uint32_t r2 = kDsNone, closer = 0;
         for (uint32_t e = e0; e < e1 && quota > 0; e += 32) {
             bool in = false;
@@ -2241,7 +2302,8 @@ __global__ void __launch_bounds__(kEvThreads) k_ds_partial(EvArgs A) {
                 uint32_t rid = A.evals[e + lane];
                 if (rid >= (uint32_t)bt.N) rid = 0;
                 m = A.ray_a[rid];
-                in = ds_is_neighbor(x, y, z, acs, m, sd.wr2);
+                in = ds_is_neighbor(x, y, z, acs, m, sd.wr2) &&
+                     (!ds_extreme(m.w) || ds_reaches_sub_block(qx, qy, qz, m, hres, sd.cull_ls2));
             }
             const unsigned mask = __ballot_sync(0xffffffffu, in);
             if (in && __popc(mask & below) < quota) {
