@@ -416,10 +416,10 @@ cudaError_t alloc_ray_buffers(k3dom_handle* h) {
         return e;
     if (h->ds()) {
         h->ds_sized_chunk = std::max(32, h->chunk);
-        const long items_max = T + cap / h->ds_sized_chunk + 2;
         rb.ds_stride = 1;
         for (const SceneHost& x : h->sc) rb.ds_stride = std::max(rb.ds_stride, x.ts.tx * x.ts.ty * x.ts.tz);
-        rb.ds_capacity = items_max * rb.ds_stride;
+        rb.ds_spare = (int)ds_spare_items(cap, h->ds_sized_chunk, rb.ds_stride);
+        rb.ds_capacity = ((long)T + rb.ds_spare + 1) * rb.ds_stride;
         if ((e = h->alloc(&rb.ds_counts, rb.ds_capacity, false, L)) || (e = h->alloc(&rb.ds_r2, rb.ds_capacity, false, L)))
             return e;
     }

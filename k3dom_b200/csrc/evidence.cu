@@ -389,17 +389,24 @@ __global__ void k_tile_start(const uint32_t* __restrict__ skeys, const uint32_t*
 // balance (30,000 rays: 111 and 128 us); 32 or 128 rays at least measured the same.
 constexpr int kItemsPerSlot = 2;
 constexpr int kItemMin = 64;
-__device__ __forceinline__ int item_rays(uint32_t entries, int chunk, int slots) {
+//
+// DS (spare > 0): chunk rays, or as many as keep the items beyond one per tile within `spare`, which
+// the per-(item, cell) summaries are sized for (ds_spare_items). The first-100 rule holds for any size.
+__device__ __forceinline__ int item_rays(uint32_t entries, int chunk, int slots, int spare) {
+    if (spare > 0) {
+        const int n = (int)(entries / (uint32_t)spare) + 1;
+        return n <= chunk ? chunk : (n + 31) & ~31;
+    }
     if (slots <= 0) return chunk;
     const uint32_t n = entries / (uint32_t)(slots * kItemsPerSlot);
     return min(chunk, max(kItemMin, (int)((n + 31u) & ~31u)));
 }
 
 __global__ void k_tile_items(const uint32_t* __restrict__ tile_start, const uint32_t* __restrict__ total, int T,
-                             int max_chunk, int slots, uint32_t* __restrict__ items) {
+                             int max_chunk, int slots, int spare, uint32_t* __restrict__ items) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
-    const int chunk = item_rays(total[2], max_chunk, slots);
+    const int chunk = item_rays(total[2], max_chunk, slots, spare);
     const uint32_t len = tile_start[t + 1] - tile_start[t];
     items[t] = len == 0 ? 1u : (len + chunk - 1) / chunk;
 }
@@ -424,7 +431,7 @@ __global__ void k_finish_lists(const uint32_t* __restrict__ item_off, int T, Dev
 // tiles. On overflow (more entries than the list holds) every range is empty.
 constexpr int kRangeThreads = 1024;
 __global__ void __launch_bounds__(kRangeThreads)
-    k_tile_ranges(uint32_t* __restrict__ tile_tally, int T, int max_chunk, int slots, long capacity,
+    k_tile_ranges(uint32_t* __restrict__ tile_tally, int T, int max_chunk, int slots, int spare, long capacity,
                   uint32_t* __restrict__ tile_start,
                   uint32_t* __restrict__ item_off, uint32_t* __restrict__ total, DevStatus* status) {
     __shared__ unsigned long long sm[kRangeThreads / 32 + 1];
@@ -435,7 +442,7 @@ __global__ void __launch_bounds__(kRangeThreads)
     unsigned long long entries;
     const unsigned long long base = block_exclusive_scan<unsigned long long, kRangeThreads>(n, sm, &entries);
     const bool over = entries > (unsigned long long)capacity;
-    const int chunk = item_rays(over ? 0u : (uint32_t)entries, max_chunk, slots);
+    const int chunk = item_rays(over ? 0u : (uint32_t)entries, max_chunk, slots, spare);
     unsigned long long o = over ? 0ull : base;
     unsigned long long ni = 0;
     for (int t = t0; t < t1; ++t) {
@@ -626,6 +633,11 @@ __global__ void k_mark_groups(uint32_t* __restrict__ groups, int ngroups, int T,
     tile_tally[t] = run;
 }
 
+long ds_spare_items(long capacity, int chunk, int stride) {
+    const long full = capacity / chunk + 1, kept = std::max(full / kDsSpareDiv, kDsSpareBytes / (5L * stride));
+    return std::min({full, kept, 0x7FFFFFFFL});
+}
+
 int mark_blocks(int N) { return std::max(1, div_up(N, kMarkRays)); }
 int mark_groups(int N) { return div_up(mark_blocks(N), kMarkGroup); }
 
@@ -693,7 +705,7 @@ cudaError_t build_ray_lists(const Batch& bt, const float* xs, const float* ys, c
         k_ds_mark<false><<<blocks, kMarkRays * kRayThreads, marks, st>>>(bt, xs, ys, zs, rb.ray_a, rb.ray_c, rb.block_base,
                                                                          rb.mark_groups, nullptr, nullptr, nullptr, status);
         k_mark_groups<<<div_up(T, 64), 64, 0, st>>>(rb.mark_groups, groups, T, rb.tile_tally);
-        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.capacity, rb.tile_start,
+        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.ds_spare, rb.capacity, rb.tile_start,
                                                    rb.item_off, rb.total, status);
         k_ds_mark<true><<<blocks, kMarkRays * kRayThreads, marks, st>>>(bt, xs, ys, zs, rb.ray_a, rb.ray_c, rb.block_base,
                                                                         rb.mark_groups, rb.tile_start, rb.total, rb.evals2,
@@ -707,7 +719,7 @@ cudaError_t build_ray_lists(const Batch& bt, const float* xs, const float* ys, c
         k_ray_count<true><<<blocks, kBlock, hist, st>>>(bt, xs, ys, zs, 0, rb.ray_a, rb.ray_c, rb.counts,
                                                          rb.tile_tally, rb.block_base, status);
         ++g_launches;
-        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.capacity, rb.tile_start,
+        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.ds_spare, rb.capacity, rb.tile_start,
                                                    rb.item_off, rb.total, status);
         ++g_launches;
         k_ray_place<<<blocks, kBlock, hist, st>>>(bt, rb.ray_a, rb.counts, rb.tile_start, rb.block_base, rb.total,
@@ -735,7 +747,8 @@ cudaError_t build_ray_lists(const Batch& bt, const float* xs, const float* ys, c
     ++g_launches;
     k_tile_start<<<div_up(T + 1, kBlock), kBlock, 0, st>>>(rb.ekeys2, rb.total, T, rb.tile_start);
     ++g_launches;
-    k_tile_items<<<div_up(T, kBlock), kBlock, 0, st>>>(rb.tile_start, rb.total, T, rb.chunk, rb.item_slots, rb.tile_items);
+    k_tile_items<<<div_up(T, kBlock), kBlock, 0, st>>>(rb.tile_start, rb.total, T, rb.chunk, rb.item_slots, rb.ds_spare,
+                                                        rb.tile_items);
     e = scan_u32_exclusive(rb.tile_items, rb.item_off, T, rb.scan_tmp, rb.item_off + T, st);
     if (e != cudaSuccess) return e;
     ++g_launches;
@@ -810,7 +823,7 @@ struct EvArgs {
     const float4* ray_a;
     const double4* ray_c;
     const uint32_t* total;  // [2]: entries in the lists
-    int item_slots;         // see item_rays
+    int item_slots, ds_spare;  // see item_rays
     uint32_t* tile_done;
     unsigned long long* acc;
     uint32_t* ds_r2;
@@ -1707,7 +1720,7 @@ __device__ __forceinline__ void run_items(const EvArgs& A, unsigned char* smem, 
     const BgkiSmem S = bgki_smem(smem, A.chunk);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t total_items = A.item_off[A.bt.T];
-    const int chunk = item_rays(A.total[2], A.chunk, A.item_slots);
+    const int chunk = item_rays(A.total[2], A.chunk, A.item_slots, 0);
     for (;;) {
         if (wid == 0) fetch_item(A, total_items, chunk, &I);
         if (threadIdx.x < kRegions) s_rcnt[threadIdx.x] = 0;
@@ -1924,7 +1937,7 @@ __device__ __forceinline__ float ds_pocc(float r_sqr, float delta) {
 constexpr int kMaxTileCells = 16 * 16 * 8;
 constexpr uint32_t kDsNone = 0xFFFFFFFFu;
 constexpr uint32_t kDsCloser = 0x10000u;  // in a cell's counter: neighbours | closer ones << 16
-static_assert(kChunk < 0x10000, "an item's count fits 16 bits");
+static_assert(kDsSpareDiv * kChunk + 64 < 0x10000, "an item's count fits 16 bits");
 
 // Per-cell results in the evidence accumulators' memory (4 words per cell).
 struct DsCells {
@@ -2098,9 +2111,10 @@ __global__ void __launch_bounds__(kEvThreads) k_ds_rays(EvArgs A) {
     const Batch& bt = A.bt;
     const DsCells D(A);
     const uint32_t total_items = A.item_off[bt.T];
+    const int chunk = item_rays(A.total[2], A.chunk, 0, A.ds_spare);
     unsigned nev = 0;  // neighbours accepted in the cells this thread finished (the roofline's work count)
     for (;;) {
-        if (wid == 0) fetch_item(A, total_items, A.chunk, &I);
+        if (wid == 0) fetch_item(A, total_items, chunk, &I);
         __syncthreads();
         if (!I.live) break;
         const TileShape ts = I.ts;
@@ -2266,6 +2280,7 @@ __global__ void __launch_bounds__(kEvThreads) k_ds_partial(EvArgs A) {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     const uint32_t n = A.status->work_counter2;
+    const uint32_t chunk = (uint32_t)item_rays(A.total[2], A.chunk, 0, A.ds_spare);
     for (uint32_t w = blockIdx.x * kEvWarps + (threadIdx.x >> 5); w < n; w += gridDim.x * kEvWarps) {
         const int c = (int)D.work_cell[w];
         const uint32_t item = D.work_item[w];
@@ -2287,8 +2302,8 @@ __global__ void __launch_bounds__(kEvThreads) k_ds_partial(EvArgs A) {
         float x, y, z;
         centre_xyz(ix, iy, iz, sd.p, fp.sensor_x, fp.sensor_y, fp.sensor_z, &x, &y, &z);
         const float acs = __fadd_rn(__fadd_rn(__fmul_rn(x, x), __fmul_rn(y, y)), __fmul_rn(z, z));
-        const uint32_t e0 = A.tile_start[t] + (item - first) * (uint32_t)A.chunk;
-        const uint32_t e1 = min(A.tile_start[t + 1], e0 + (uint32_t)A.chunk);
+        const uint32_t e0 = A.tile_start[t] + (item - first) * chunk;
+        const uint32_t e1 = min(A.tile_start[t + 1], e0 + chunk);
         const float hres = 0.5f * sd.p.res;
         float qx, qy, qz;  // centroid of the cell's sub-block
         centre_xyz((ix & ~3) + 2, (iy & ~3) + 2, (iz & ~1) + 1, sd.p, fp.sensor_x, fp.sensor_y, fp.sensor_z, &qx, &qy,
@@ -2357,6 +2372,7 @@ static EvArgs make_args(const Batch& bt, RayBuffers& rb, CellState cs, CellWork 
     A.ray_c = rb.ray_c;
     A.total = rb.total;
     A.item_slots = rb.item_slots;
+    A.ds_spare = rb.ds_spare;
     A.tile_done = rb.tile_done;
     A.acc = rb.acc;
     A.ds_r2 = rb.ds_r2;

@@ -170,6 +170,7 @@ struct RayBuffers {
     long capacity;         // entries
     long ds_capacity;      // DS: (item, cell) summaries
     int ds_stride;         // DS: cells of the largest tile
+    int ds_spare;          // DS: items beyond one per tile that the summaries are sized for (0: K3DOM)
     int chunk;             // largest number of rays per work item
     int item_slots;        // CTA slots the work items are spread over (0: items of chunk rays whatever the scene)
 };
@@ -190,6 +191,15 @@ int mark_groups(int N);
 inline bool placed_lists(bool ds, int T, int N) {
     return ds ? T <= kMarkMaxTiles && (long)mark_blocks(N) * T <= kMarkMaxCounts : T <= kPlacedMaxTiles;
 }
+// DS summaries take 5 bytes per (item, cell), and the items of chunk rays that lists at their capacity
+// would make need far more of them than frames do (256x256x32 voxels, 120,000 rays: capacity 23.0M
+// entries, 2.3M held). A tenth of those items is allowed for, 64 MB at least; a frame with more entries
+// than that makes larger items (item_rays), up to kDsSpareDiv times the chunk. The handle there takes
+// 520 MB instead of 912 (items of 512 rays) and 1.2 GB instead of 7.8 (32 rays), at the same frame time
+// (837 and 838 us).
+constexpr int kDsSpareDiv = 10;
+constexpr long kDsSpareBytes = 64L << 20;
+long ds_spare_items(long capacity, int chunk, int stride);
 constexpr int kBinBlocksMax = 1024;
 int bin_blocks(long n);  // blocks of the placed-list passes over n threads
 constexpr int kRayThreads = 2;  // threads per ray in the placed-list passes
