@@ -405,7 +405,7 @@ cudaError_t alloc_ray_buffers(k3dom_handle* h) {
     cap = std::max(cap, 4096L);
     if (cap > 0xFFFFFFF0L) cap = 0xFFFFFFF0L;
     rb.capacity = cap;
-    rb.chunk = h->chunk;
+    rb.chunk = evidence_chunk(h->ds(), h->chunk);
     rb.item_slots = h->ds() ? 0 : evidence_slots(h->num_sms);
     const int N = h->N, T = h->T;
     if ((e = h->alloc(&rb.ray_a, N, true, L)) || (e = h->alloc(&rb.ray_c, N, true, L)) ||
@@ -913,7 +913,7 @@ cudaError_t apply_tuning(k3dom_handle* h, int rule, int chunk) {
         if (e == cudaSuccess) e = cudaEventRecord(h->ev_staged, h->st);
         return e;
     }
-    h->rb.chunk = chunk;
+    h->rb.chunk = evidence_chunk(h->ds(), chunk);
     return cudaSuccess;
 }
 

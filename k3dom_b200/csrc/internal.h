@@ -174,6 +174,13 @@ struct RayBuffers {
     int chunk;             // largest number of rays per work item
     int item_slots;        // CTA slots the work items are spread over (0: items of chunk rays whatever the scene)
 };
+// Rays per work item for a tuned chunk: K3DOM takes kItemLeast at least (fewer leave its batches of 32
+// candidates per class part empty, and every sub-block's set-up is paid per item). A frame of
+// 256x256x32 voxels, 120,000 rays, 16x16x8 tiles, by chunk: 32 rays 5,725 us, 64 3,523, 128 2,406, 256
+// 1,778 (one cell a lane without batches: 3,829, 2,921, 2,487, 2,294); 64x64x16, 30,000 rays, 8x8x4
+// tiles: 358, 273, 229, 214 (269, 237, 218, 220).
+constexpr int kItemLeast = 256;
+inline int evidence_chunk(bool ds, int chunk) { return ds || chunk > kItemLeast ? chunk : kItemLeast; }
 long ray_entries_bound(const DevParams& p, const TileShape& ts, int max_points, float bin_R);
 // Ray lists are placed per tile through block histograms (K3DOM: 4 bytes a tile) or bit masks (DS: 16
 // bytes) of all T tiles in shared memory; otherwise the entries are sorted by tile. Both take what
