@@ -1422,6 +1422,11 @@ __device__ __forceinline__ TabPos2 tab_pos2(F2 d2, F2 tscale) {
 constexpr float kFxHi = 6.0f;                    // [4, 8): ulp 2^-21
 constexpr float kFxLo = 1.5f / (1 << 17);        // [2^-17, 2^-16): ulp 2^-40
 constexpr uint32_t kFxHiBits = 0x40C00000u, kFxLoBits = 0x37400000u;
+constexpr int kFxMost = 2047, kFxMostSigned = 1023;
+// Values a sub-block adds per cell: the item's rays, and up to 7 pads in the last batch of each class.
+constexpr int kFxPads = 14;
+static_assert(kChunk + kFxPads <= kFxMost, "K3DOM sums");
+static_assert(kCalibChunk + kFxPads <= kFxMostSigned, "calibration sums: the derivative's are signed");
 
 struct FxSum {
     uint32_t hi, lo;
@@ -1435,8 +1440,8 @@ struct FxSum {
         hi += __float_as_uint(ta) + __float_as_uint(tb);
         lo += __float_as_uint(qa) + __float_as_uint(qb);
     }
-    // The sum of n added values, in units; at most 2,047 values in [0, 1] (total), or 1,023 in
-    // [-1, 1] (total_signed), and kChunk plus a pad is fewer.
+    // The sum of n added values, in units; at most kFxMost values in [0, 1] (total), or kFxMostSigned in
+    // [-1, 1] (total_signed): the high parts, at most 2^21 each, add up in 32 bits.
     __device__ __forceinline__ long long total(uint32_t n) const {
         return ((long long)(uint32_t)(hi - n * kFxHiBits) << 19) + (int32_t)(lo - n * kFxLoBits);
     }
