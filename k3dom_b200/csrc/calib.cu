@@ -726,7 +726,7 @@ k3dom_status k3dom_calib_create(const k3dom_params* base, int device, k3dom_cali
     cudaDeviceProp prop;
     if ((e = cudaGetDeviceProperties(&prop, device))) return bail(e);
     c->num_sms = prop.multiProcessorCount;
-    if ((e = sort_init()) || (e = evidence_init())) return bail(e);
+    if ((e = evidence_init())) return bail(e);
     DevParams& d = c->dp;
     d.G = static_cast<int>(base->size / base->resolution);
     d.Gz = static_cast<int>(base->size_z / base->resolution);

@@ -984,7 +984,7 @@ k3dom_status k3dom_batch_create(const k3dom_params* params, int32_t n_scenes, k3
     cudaDeviceProp prop;
     if ((e = cudaGetDeviceProperties(&prop, device))) return bail(e);
     h->num_sms = prop.multiProcessorCount;
-    if ((e = sort_init()) || (e = onesweep_init()) || (e = evidence_init())) return bail(e);
+    if ((e = onesweep_init()) || (e = evidence_init())) return bail(e);
 
     // scene ranges
     int P = 0, B = 0, C = 0;

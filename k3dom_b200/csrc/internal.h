@@ -13,27 +13,10 @@ namespace k3dom {
 // across it). Handles are single-threaded, as the reference's DOM is.
 extern long g_launches;
 
-// sort.cu
+// scan.cu
 int scan_u32_tiles(long n);
-cudaError_t scan_u32_exclusive(const uint32_t* in, uint32_t* out, long n, uint32_t* tmp,
-                               uint32_t* total, cudaStream_t st);
-// Same with the element count min(*dn, nmax) read on the device (dn may be nullptr).
-cudaError_t scan_u32_exclusive_dn(const uint32_t* in, uint32_t* out, long nmax, const uint32_t* dn,
-                                  uint32_t* tmp, uint32_t* total, cudaStream_t st);
-int radix_tiles(long n);
-long radix_hist_words(long n, int max_bits);
-int radix_plan(int key_bits, int* pass_bits);
-// hist_words / scan_words are the capacities of hist and scan_tmp (radix_hist_words(n, 11) and
-// scan_u32_tiles of it suffice for any key width); too small a buffer is refused.
-cudaError_t radix_sort_pairs(const uint32_t* keys, const uint32_t* vals, uint32_t* keys_out,
-                             uint32_t* vals_out, uint32_t* alt_k, uint32_t* alt_v, long n,
-                             int key_bits, uint32_t* hist, long hist_words, uint32_t* scan_tmp,
-                             long scan_words, cudaStream_t st);
-cudaError_t radix_sort_pairs_dn(const uint32_t* keys, const uint32_t* vals, uint32_t* keys_out,
-                                uint32_t* vals_out, uint32_t* alt_k, uint32_t* alt_v, long nmax,
-                                const uint32_t* dn, int key_bits, uint32_t* hist, long hist_words,
-                                uint32_t* scan_tmp, long scan_words, cudaStream_t st);
-cudaError_t sort_init();
+cudaError_t scan_u32_exclusive(const uint32_t* in, uint32_t* out, long n, uint32_t* tmp, uint32_t* total,
+                               cudaStream_t st);
 
 // onesweep.cu: the particle sort (one histogram read, then one read and write per 7-bit digit
 // with decoupled look-back). A look-back poll loop gives up after max_polls polls and sets

@@ -18,12 +18,11 @@
 //    look-back, so later tiles count past it), so the output holds the keys and values of the
 //    completed tiles and in-range old contents elsewhere; the later passes then write nothing.
 // Digits of up to 8 bits, a key of b bits taking ceil(b / 8) passes of (nearly) equal width:
-// the 21-bit cell keys of 2^21 voxels three passes of 7 bits;
-// up to 256 digits per tile keep the runs long enough for coalesced writes. The element count
-// may live in device memory (`dn`, capped at nmax): the grid and scratch are sized for nmax,
-// CTAs whose tile lies past the live count return, and since tiles are handed out in order no
-// CTA waits on one of them. The same
-// sort orders the ray lists (tile of each entry, stable so each tile keeps its rays in input order).
+// the 21-bit cell keys of 2^21 voxels three passes of 7 bits; up to 256 digits per tile keep the runs
+// long enough for coalesced writes. The element count may live in device memory (`dn`, capped at
+// nmax): the grid and scratch are sized for nmax, CTAs whose tile lies past the live count return, and
+// since tiles are handed out in order no CTA waits on one of them. The same sort orders sorted ray
+// lists (tile of each entry, stable so each tile keeps its rays in input order).
 #include <cuda_runtime.h>
 
 #include <algorithm>
