@@ -408,8 +408,10 @@ cudaError_t alloc_ray_buffers(k3dom_handle* h) {
     rb.chunk = evidence_chunk(h->ds(), h->chunk);
     rb.item_slots = h->ds() ? 0 : evidence_slots(h->num_sms);
     const int N = h->N, T = h->T;
-    if ((e = h->alloc(&rb.ray_a, N, true, L)) || (e = h->alloc(&rb.ray_c, N, true, L)) ||
-        (e = h->alloc(&rb.counts, (size_t)kRayThreads * N, true, L)) || (e = h->alloc(&rb.evals2, cap, false, L)) ||
+    const bool placed = placed_lists(h->ds(), T, N);
+    if ((e = h->alloc(&rb.ray_a, N, true, L)) || (!h->ds() && (e = h->alloc(&rb.ray_c, N, true, L))) ||
+        (!(h->ds() && placed) && (e = h->alloc(&rb.counts, (size_t)kRayThreads * N, true, L))) ||
+        (e = h->alloc(&rb.evals2, cap, false, L)) ||
         (e = h->alloc(&rb.tile_start, T + 1, true, L)) || (e = h->alloc(&rb.item_off, T + 1, true, L)) ||
         (e = h->alloc(&rb.tile_done, T, true, L)) || (e = h->alloc(&rb.acc, 2 * (size_t)h->C, true, L)) ||
         (e = h->alloc(&rb.total, 4, true, L)))
@@ -423,7 +425,7 @@ cudaError_t alloc_ray_buffers(k3dom_handle* h) {
         if ((e = h->alloc(&rb.ds_counts, rb.ds_capacity, false, L)) || (e = h->alloc(&rb.ds_r2, rb.ds_capacity, false, L)))
             return e;
     }
-    if (placed_lists(h->ds(), T, N)) {  // per-tile tallies and per-block offsets or counts
+    if (placed) {  // per-tile tallies and per-block offsets or counts
         const long blocks = h->ds() ? mark_blocks(N) : bin_blocks((long)kRayThreads * N);
         if ((e = h->alloc(&rb.tile_tally, T, true, L)) || (e = h->alloc(&rb.block_base, (size_t)blocks * T, true, L)) ||
             (h->ds() && (e = h->alloc(&rb.mark_groups, (size_t)mark_groups(N) * T, true, L))))

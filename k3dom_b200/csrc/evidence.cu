@@ -296,7 +296,7 @@ __global__ void k_ray_count(Batch bt, const float* __restrict__ xs, const float*
         const RayPrep r = prep_ray(sd.p, g, mx, my, mz, ds != 0, &a, &cc, half == 0);
         if (half == 0) {
             ra[i] = a;
-            rc[i] = cc;
+            if (!ds) rc[i] = cc;
         }
         uint32_t c = 0;
         if (r.ok) {
@@ -542,8 +542,8 @@ constexpr int kMarkWords = kMarkRays / 32;
 template <bool PLACE>
 __global__ void __launch_bounds__(kMarkRays * kRayThreads)
 k_ds_mark(Batch bt, const float* __restrict__ xs, const float* __restrict__ ys, const float* __restrict__ zs,
-          float4* __restrict__ ra, double4* __restrict__ rc, uint32_t* __restrict__ rows,
-          uint32_t* __restrict__ groups, const uint32_t* __restrict__ tile_start, const uint32_t* __restrict__ total,
+          float4* __restrict__ ra, uint32_t* __restrict__ rows, uint32_t* __restrict__ groups,
+          const uint32_t* __restrict__ tile_start, const uint32_t* __restrict__ total,
           uint32_t* __restrict__ evals, DevStatus* status) {
     extern __shared__ uint4 s_mark[];  // [T]: the block's rays that reach the tile
     static_assert(kMarkWords == 4, "one uint4 per tile");
@@ -564,10 +564,7 @@ k_ds_mark(Batch bt, const float* __restrict__ xs, const float* __restrict__ ys, 
         float4 a;
         double4 c;
         const RayPrep p = prep_ray(sd.p, g, mx, my, mz, true, &a, &c);
-        if (!PLACE && half == 0) {
-            ra[i] = a;
-            rc[i] = c;
-        }
+        if (!PLACE && half == 0) ra[i] = a;
         if (p.ok) {
             uint32_t* word = reinterpret_cast<uint32_t*>(s_mark + bt.off->tile[sc]) + (r >> 5);
             const uint32_t bit = 1u << (r & 31);
@@ -702,14 +699,13 @@ cudaError_t build_ray_lists(const Batch& bt, const float* xs, const float* ys, c
         cudaError_t e = cudaMemsetAsync(rb.mark_groups, 0, sizeof(uint32_t) * (size_t)groups * T, st);
         if (e != cudaSuccess) return e;
         g_launches += 4;
-        k_ds_mark<false><<<blocks, kMarkRays * kRayThreads, marks, st>>>(bt, xs, ys, zs, rb.ray_a, rb.ray_c, rb.block_base,
-                                                                         rb.mark_groups, nullptr, nullptr, nullptr, status);
+        k_ds_mark<false><<<blocks, kMarkRays * kRayThreads, marks, st>>>(
+            bt, xs, ys, zs, rb.ray_a, rb.block_base, rb.mark_groups, nullptr, nullptr, nullptr, status);
         k_mark_groups<<<div_up(T, 64), 64, 0, st>>>(rb.mark_groups, groups, T, rb.tile_tally);
-        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.ds_spare, rb.capacity, rb.tile_start,
-                                                   rb.item_off, rb.total, status);
-        k_ds_mark<true><<<blocks, kMarkRays * kRayThreads, marks, st>>>(bt, xs, ys, zs, rb.ray_a, rb.ray_c, rb.block_base,
-                                                                        rb.mark_groups, rb.tile_start, rb.total, rb.evals2,
-                                                                        status);
+        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.ds_spare, rb.capacity,
+                                                   rb.tile_start, rb.item_off, rb.total, status);
+        k_ds_mark<true><<<blocks, kMarkRays * kRayThreads, marks, st>>>(
+            bt, xs, ys, zs, rb.ray_a, rb.block_base, rb.mark_groups, rb.tile_start, rb.total, rb.evals2, status);
         return cudaGetLastError();
     }
     if (placed_lists(ds, T, N)) {  // K3DOM: tally, ranges, place
@@ -719,8 +715,8 @@ cudaError_t build_ray_lists(const Batch& bt, const float* xs, const float* ys, c
         k_ray_count<true><<<blocks, kBlock, hist, st>>>(bt, xs, ys, zs, 0, rb.ray_a, rb.ray_c, rb.counts,
                                                          rb.tile_tally, rb.block_base, status);
         ++g_launches;
-        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.ds_spare, rb.capacity, rb.tile_start,
-                                                   rb.item_off, rb.total, status);
+        k_tile_ranges<<<1, kRangeThreads, 0, st>>>(rb.tile_tally, T, rb.chunk, rb.item_slots, rb.ds_spare, rb.capacity,
+                                                   rb.tile_start, rb.item_off, rb.total, status);
         ++g_launches;
         k_ray_place<<<blocks, kBlock, hist, st>>>(bt, rb.ray_a, rb.counts, rb.tile_start, rb.block_base, rb.total,
                                                    rb.evals2);

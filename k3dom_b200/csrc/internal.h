@@ -125,7 +125,8 @@ struct RayBuffers {
     double4* ray_c;        // d_m, margin, 1/d_m, 0 in FP64 (K3DOM)
     float4* ktab;          // per scene: sparse-kernel table with the fixed-point scale folded in
     cudaTextureObject_t ktex;  // the kernel table through the texture path (k_bgki: ktab; k_bgki_sums: f), 0 when not made
-    uint32_t* counts;      // [kRayThreads * N] tiles touched per point slot (DS) or per thread of a slot
+    uint32_t* counts;      // [kRayThreads * N] tiles touched per point slot (sorted lists) or per thread of a slot
+                           // (placed K3DOM lists)
     uint32_t* offsets;     // exclusive scan of counts (sorted lists)
     uint32_t* ekeys;       // entries: global tile id (sorted lists)
     uint32_t* evals;       // entries: point slot (sorted lists)
