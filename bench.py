@@ -396,6 +396,14 @@ def measure_plain(args, variant: str, cfg, rank: int, world: int, local: int, di
         dom.close()
 
 
+def tiling_name(rule: int, variant: str, cells: int) -> str:
+    """The tiles of an evidence rule; rule 0 chooses by variant and size (tile_shape in csrc/dom.cu)."""
+    if rule == 0:
+        ds = variant != "k3dom"
+        rule = (3 if ds else 2) if cells >= (1 << 17 if ds else 1 << 19) else 1
+    return ["", "8x8x4", "16x16x4", "16x16x8"][rule]
+
+
 def evidence_roofline(m: dict, variant: str) -> dict:
     """The dominant kernel's line: in-support evaluations (K3DOM) or accepted neighbours (DS) x
     FLOP per unit / its CUDA-event time / the nominal FP32 issue peak."""
@@ -405,9 +413,7 @@ def evidence_roofline(m: dict, variant: str) -> dict:
     achieved = m["evals"] * flop_per / (ev_ms * 1e-3) / 1e12
     traffic, issue = None, None
     tr_file = ROOT / "profiles" / ("dsgrid_traffic.json" if ds else "bgki_traffic.json")
-    rule_name = ["by-size", "8x8x4", "16x16x4", "16x16x8"][m["tuning"]["tile_rule"]]
-    if rule_name == "by-size":
-        rule_name = "16x16x4"  # the rule's choice for K3DOM grids of >= 2^19 cells
+    rule_name = tiling_name(m["tuning"]["tile_rule"], variant, m["C"])
     if tr_file.exists():
         try:
             d = json.loads(tr_file.read_text())
