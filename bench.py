@@ -412,9 +412,9 @@ def evidence_roofline(m: dict, variant: str) -> dict:
     flop_per = FLOP_PER_DS_NEIGHBOUR if ds else FLOP_PER_EVAL
     achieved = m["evals"] * flop_per / (ev_ms * 1e-3) / 1e12
     traffic, issue = None, None
-    tr_file = ROOT / "profiles" / ("dsgrid_traffic.json" if ds else "bgki_traffic.json")
+    tr_file = ROOT / "profiles" / "bgki_traffic.json"  # K3DOM only
     rule_name = tiling_name(m["tuning"]["tile_rule"], variant, m["C"])
-    if tr_file.exists():
+    if not ds and tr_file.exists():
         try:
             d = json.loads(tr_file.read_text())
             issue = d.get("issue")

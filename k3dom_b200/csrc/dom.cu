@@ -43,10 +43,19 @@ enum TileRule { kRuleBySize = 0, kRuleSmall = 1, kRuleFlat = 2, kRuleLarge = 3, 
 TileShape tile_shape(const DevParams& p, int rule) {
     int tx = 8, ty = 8, tz = 4;
     // By size: larger tiles mean fewer list entries and fewer items, smaller ones more items for the
-    // GPU's slots. Frames in us with 8x8x4, 16x16x4, 16x16x8 tiles (0.1 to 0.2 m voxels, 60,000 and
-    // 120,000 rays): K3DOM 250k cells 447, 454, 480; 524k 652, 659, 718 and (0.2 m) 441, 433, 475; 1M
-    // 625, 621, 657; 1.05M 1138, 1083, 1168; 2.1M 1564, 1471, 1567; 3.2M 1118, 965, 1050. DS 250k 346,
-    // 327, 321; 524k 429, 412, 405; 1M 476, 434, 412; 2.1M 871, 766, 733.
+    // GPU's slots. Frames in us with 8x8x4, 16x16x4, 16x16x8 tiles (1M particles; ls 0.3 m at 0.1 m
+    // voxels and 0.5 m at 0.2 m but for the first):
+    //   K3DOM 100x100x25 at 0.2 m, ls 0.3 m, 60,000 rays   387, 381, 413
+    //         160x160x20 at 0.2 m, 60,000                  583, 576, 623
+    //         128x128x32 at 0.1 m, 60,000                  665, 677, 732
+    //         200x200x25 at 0.2 m, 60,000                  634, 631, 665
+    //         256x256x16 and x32 at 0.1 m, 120,000         1045, 1024, 1096 and 1491, 1397, 1499
+    //         400x400x20 at 0.1 m, 120,000                 1497, 1315, 1449
+    //   DS    64x64x16 at 0.2 m, 30,000                    258, 265, 262
+    //         100x100x12 and x25 at 0.2 m, 60,000          313, 308, 301 and 338, 335, 327
+    //         128x128x32 at 0.1 m, 60,000                  381, 360, 349
+    //         200x200x25 at 0.2 m, 60,000                  437, 391, 378
+    //         256x256x32 at 0.1 m, 120,000                 774, 604, 590
     const bool large = (long)p.C >= (p.variant != 0 ? 1L << 17 : 1L << 19);
     switch (rule) {
         case kRuleBySize:
@@ -172,7 +181,7 @@ struct k3dom_handle {
 
     // evidence tuning
     int tile_rule = kRuleBySize;
-    int chunk = 1024;        // DS starts at 512 (200x200x25 voxels 412 -> 396 us, 2.1M cells equal)
+    int chunk = 1024;        // DS starts at 512 (200x200x25 voxels 412 -> 396 us, 256x256x32 equal)
     int tune_next = -1;  // next candidate to measure, -1 when not tuning
     float tune_best_ms = 0.0f;
     int tune_best = 0, tuned = 0;

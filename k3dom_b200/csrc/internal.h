@@ -168,10 +168,10 @@ inline int evidence_chunk(bool ds, int chunk) { return ds || chunk > kItemLeast 
 long ray_entries_bound(const DevParams& p, const TileShape& ts, int max_points, float bin_R);
 // Ray lists are placed per tile through block histograms (K3DOM: 4 bytes a tile) or bit masks (DS: 16
 // bytes) of all T tiles in shared memory; otherwise the entries are sorted by tile. Both take what
-// lets two blocks share an SM. K3DOM batches of 4 to 11 uneven scenes, lists placed and sorted: 12,736
-// tiles 359 and 743 us, 17,429 574 and 1,112, 27,293 1,028 and 1,561, 36,449 (one block per SM) 2,212
-// and 2,108. DS, 256x256x32 voxels, 120,000 rays: 1,024 tiles 76 and 145 us, 2,048 94 and 156, 8,192
-// (one block) 271 and 229. DS keeps up to kMarkMaxCounts counts (128 MB).
+// lets two blocks share an SM. K3DOM, 1 to 4 scenes of 256x256x32 voxels at 0.1 m and 120,000 rays in
+// 8x8x4 tiles, lists placed and sorted: 8,192 tiles 177 and 400 us, 16,384 344 and 655, 24,576 638 and
+// 894, 32,768 (one block per SM) 1,439 and 1,154. DS, one such scene: 1,024 tiles 76 and 145 us, 2,048
+// 94 and 156, 8,192 (one block) 271 and 229. DS keeps up to kMarkMaxCounts counts (128 MB).
 constexpr int kPlacedMaxTiles = 28416;
 constexpr int kMarkMaxTiles = 6144;
 constexpr int kMarkRays = 128;   // rays per block of the DS passes
