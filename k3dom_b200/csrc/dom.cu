@@ -1374,9 +1374,7 @@ k3dom_status k3dom_update_grid_async(k3dom_handle* h, float t, const float* xs, 
 k3dom_status k3dom_synchronize(k3dom_handle* h) {
     if (!h) return K3DOM_ERR_INVALID_ARGUMENT;
     cudaSetDevice(h->device);
-    k3dom_status s = finish_sync(h);
-    if (s == K3DOM_OK && h->timing) read_times(h);
-    return s;
+    return finish_sync(h);  // a timed frame has waited and read its times itself
 }
 
 k3dom_status k3dom_get_stream(k3dom_handle* h, void** stream) {
