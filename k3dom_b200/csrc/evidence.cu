@@ -16,11 +16,12 @@
 // (scene tile offset + local tile), so one pass builds every scene's lists. K3DOM places each
 // ray into its tiles' ranges through per-block tallies of each tile (its exact sums make the order
 // within a tile immaterial); DS keeps a tile's rays in input order, as its first-100 rule needs (bit
-// masks per block of rays, k_ds_mark); with too many tiles for either, a stable sort by tile. One CTA takes one (tile, chunk of rays) work item
-// from a device work counter and stages the chunk's rays in shared memory; its warps pull the
-// tile's 4x4x2-cell sub-blocks from a block-local counter and cull 32 rays at a time with one
-// ballot, collect the surviving rays into batches of 32, resolve them in FP64 and evaluate two rays
-// at a time for four cells per lane. DS walks each ray's cells (see k_ds_rays).
+// masks per block of rays, k_ds_mark); with too many tiles for either, a stable sort by tile. One CTA
+// takes one (tile, chunk of rays) work item from a device work counter and stages the chunk's rays in
+// shared memory; its warps pull the tile's 4x4x2-cell sub-blocks from a block-local counter and cull
+// 32 rays at a time with one ballot, collect the surviving rays into batches of 32, resolve them in
+// FP64 and evaluate two rays at a time for four cells per lane. DS walks each ray's cells (see
+// k_ds_rays).
 //
 // K3DOM evidence is summed in fixed point: each kernel value is rounded once to an integer
 // number of units of 2^-k sigma (the table carries the scale), summed exactly in 64-bit

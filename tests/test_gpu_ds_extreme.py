@@ -3,8 +3,8 @@ sensor: a sensor's marker for no return, a return at the sensor itself). The ref
 test (measurement_grid.cu:88-99) is no window around the half-line for them; csrc/evidence.cu applies it to
 every cell of the 4x4x2 sub-blocks near the half-line, formed in FP32 (ds_reaches_sub_block), in the tiles
 that the ray's binned segment meets. Here the same rule over all (cell, ray) pairs in numpy float32, with
-the first-100 rule in input order; cells whose pOcc comparison is within 4 ulp of flipping are left out, pOcc is compared to the 2.5e-7
-of expf's 2 ulp."""
+the first-100 rule in input order; cells whose pOcc comparison is within 4 ulp of flipping are left out,
+pOcc is compared to the 2.5e-7 of expf's 2 ulp."""
 import numpy as np
 import pytest
 
